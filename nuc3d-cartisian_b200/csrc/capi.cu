@@ -85,7 +85,7 @@ int read_tuning(const Engine *eng, int *run_len, double *ms) {
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d) {
             int v = eng->inv_variant[s][d];
-            if (run_len) run_len[s * 3 + d] = v < 0 ? 0 : kInvRunLen[v];
+            if (run_len) run_len[s * 3 + d] = v < 0 ? 0 : eng->sweep_run(s, d, v);
             for (int k = 0; k < 3; ++k)
                 if (ms) ms[(s * 3 + d) * 3 + k] = eng->inv_tune_ms[s][d][k];
         }
@@ -98,7 +98,7 @@ int read_tiles(const Engine *eng, int *tile_cells, double *ms64) {
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d) {
             int v = eng->inv_variant[s][d];
-            if (tile_cells) tile_cells[s * 3 + d] = v < 0 ? 0 : kInvTileCells[v];
+            if (tile_cells) tile_cells[s * 3 + d] = v < 0 ? 0 : eng->sweep_tile(s, d, v);
             for (int k = 0; k < 2; ++k)
                 if (ms64) ms64[(s * 3 + d) * 2 + k] = eng->inv_tune_ms[s][d][3 + k];
         }

@@ -441,7 +441,9 @@ int Engine::rebuild() {
     const bool mixed = precision_ == NUC3D_MIXED;
     std::vector<BoxDev> table(boxes_.size());
     std::vector<WorkItem> prim, st25[kVisClasses][3], inv[kSchemes][3][kInvTileClasses],
-        cr[kLineSchemes][3];
+        march[kSchemes][3], cr[kLineSchemes][3];
+    for (int s = 0; s < kSchemes; ++s)
+        for (int d = 0; d < 3; ++d) march_nmax_[s][d] = 0;
     const int crtl = crweno_tile_lines();
     for (int c = 0; c < kLineSchemes; ++c)
         for (int d = 0; d < 3; ++d) cr_nmax_[c][d] = cr_ms_[c][d] = 0;
@@ -488,6 +490,12 @@ int Engine::rebuild() {
                 }
                 continue;
             }
+            if (marched(s, d, mixed)) {
+                march_nmax_[s][d] = std::max(march_nmax_[s][d], p.n[d]);
+                const long long lines = p.N / p.n[d];
+                for (int g = 0; g * 32LL < lines; ++g) march[s][d].push_back({id, g, 0, 0});
+                continue;
+            }
             for (int tc = 0; tc < kInvTileClasses; ++tc) {
                 InvTileDims t = inviscid_tile(d, mixed, tc == 0 ? 32 : 64);
                 auto &L = inv[s][d][tc];
@@ -519,6 +527,8 @@ int Engine::rebuild() {
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d)
             for (int tc = 0; tc < kInvTileClasses; ++tc) append(inv[s][d][tc], r_inv_[s][d][tc]);
+    for (int s = 0; s < kSchemes; ++s)
+        for (int d = 0; d < 3; ++d) append(march[s][d], r_march_[s][d]);
     for (int c = 0; c < kLineSchemes; ++c)
         for (int d = 0; d < 3; ++d) append(cr[c][d], r_cr_[c][d]);
     if ((int)boxes_.size() > d_boxes_cap_) {
@@ -541,13 +551,14 @@ int Engine::rebuild() {
                             cudaMemcpyHostToDevice, stream_));
     ECK(cudaStreamSynchronize(stream_));  // host vectors go out of scope
     ECK(prepare_inviscid_kernels(mixed));
+    if (!mixed) ECK(prepare_march_kernels());
     ECK(prepare_crweno_kernels(mixed));
     ECK(prepare_stencil_kernels(mixed));
     int per_stage = 0;
     for (int c = 0; c < kVisClasses; ++c)
         per_stage += (any_visc_ && r_25d_[c][0].n > 0) + (r_25d_[c][0].n > 0);
     for (int s = 0; s < kSchemes; ++s)
-        for (int d = 0; d < 3; ++d) per_stage += r_inv_[s][d][0].n > 0;
+        for (int d = 0; d < 3; ++d) per_stage += has_sweep(s, d);
     for (int c = 0; c < kLineSchemes; ++c)
         for (int d = 0; d < 3; ++d) per_stage += r_cr_[c][d].n > 0;
     launches_per_step_ = 3 * per_stage + 3;  // + clear_eig, dt, residual
@@ -613,8 +624,7 @@ int Engine::enqueue_step_t(cudaStream_t st) {
             ProfScope ps(this, NUC3D_PROF_INV_X + d);
             const int prim_mode = d == 0 ? (stage == 0 ? 2 : 1) : 0;
             for (int s = 0; s < kSchemes; ++s)
-                ECK((launch_inviscid<B>(s, d, inv_variant[s][d], d_boxes_, it + inv_range(s, d).off,
-                                        inv_range(s, d).n, in, d > 0, prim_mode, st)));
+                ECK((launch_sweep<B>(s, d, inv_variant[s][d], in, prim_mode, st)));
             for (int c = 0; c < kLineSchemes; ++c)
                 ECK((launch_crweno<B>(kLineScheme[c], d, d_boxes_,
                                       it + r_cr_[c][d].off, r_cr_[c][d].n, in, d > 0,
@@ -658,6 +668,16 @@ int Engine::enqueue_step_t(cudaStream_t st) {
         ECK(launch_residual(d_boxes_, nb, st));
     }
     return NUC3D_OK;
+}
+
+template <typename B>
+cudaError_t Engine::launch_sweep(int s, int d, int v, int in, int prim_mode, cudaStream_t st) {
+    const Range &m = r_march_[s][d];
+    if (m.n > 0)
+        return launch_march(s, d, d_boxes_, d_items_ + m.off, m.n, march_nmax_[s][d], in,
+                            kMarchLen[v], st);
+    const Range &r = r_inv_[s][d][v < 0 ? 0 : inv_tile_class(v)];
+    return launch_inviscid<B>(s, d, v, d_boxes_, d_items_ + r.off, r.n, in, d > 0, prim_mode, st);
 }
 
 template <typename B>
@@ -717,7 +737,7 @@ int Engine::autotune() {
     bool need_sweep = false;
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d)
-            need_sweep = need_sweep || (r_inv_[s][d][0].n > 0 && inv_variant[s][d] < 0);
+            need_sweep = need_sweep || (has_sweep(s, d) && inv_variant[s][d] < 0);
     const bool need_pencil =
         (r_25d_[0][0].n > 0 || r_25d_[1][0].n > 0) &&
         (pencil_variant < 0 || 2 * active_cells_ < pencil_tuned_cells ||
@@ -738,7 +758,7 @@ int Engine::autotune() {
                 if (kInvRunLen[k] == run && kInvTileCells[k] == tc) v = k;
             for (int s = 0; s < kSchemes; ++s)
                 for (int d = 0; d < 3; ++d)
-                    if (r_inv_[s][d][0].n > 0 && inv_variant[s][d] < 0) inv_variant[s][d] = v;
+                    if (has_sweep(s, d) && inv_variant[s][d] < 0) inv_variant[s][d] = v;
             need_sweep = false;
         }
     }
@@ -780,23 +800,20 @@ int Engine::autotune() {
     };
     for (int s = 0; s < kSchemes && rc == NUC3D_OK && need_sweep; ++s)
         for (int d = 0; d < 3 && rc == NUC3D_OK; ++d) {
-            if (r_inv_[s][d][0].n <= 0 || inv_variant[s][d] >= 0) continue;
+            if (!has_sweep(s, d) || inv_variant[s][d] >= 0) continue;
             int best = 0;
             for (int v = 0; v < kInvVariants && rc == NUC3D_OK; ++v) {
                 if (inv_tile_class(v) == 1 && mixed_tiles_only32()) {
                     inv_tune_ms[s][d][v] = 0.0;
                     continue;
                 }
-                const Range &rg = r_inv_[s][d][inv_tile_class(v)];
                 // the x sweep is timed as the step runs it, recovering the
                 // primitives of its tiles (prim_mode 1): it rewrites W with
                 // bitwise the values k_prim has just written
                 const int pm = d == 0 ? 1 : 0;
                 const double ms = time3([&]() {
-                    return mixed ? launch_inviscid<float>(s, d, v, d_boxes_, d_items_ + rg.off, rg.n,
-                                                          0, d > 0, pm, stream_)
-                                 : launch_inviscid<double>(s, d, v, d_boxes_, d_items_ + rg.off,
-                                                           rg.n, 0, d > 0, pm, stream_);
+                    return mixed ? launch_sweep<float>(s, d, v, 0, pm, stream_)
+                                 : launch_sweep<double>(s, d, v, 0, pm, stream_);
                 });
                 inv_tune_ms[s][d][v] = ms;
                 if (ms < inv_tune_ms[s][d][best]) best = v;
@@ -914,8 +931,7 @@ int Engine::enqueue_rhs_t(int id, double *const d_rhs[5]) {
     if (any_visc_) ECK(launch_visc_classes<B>(pv(), stream_));
     for (int d = 0; d < 3; ++d) {
         for (int s = 0; s < kSchemes; ++s)
-            ECK((launch_inviscid<B>(s, d, inv_variant[s][d], d_boxes_, it + inv_range(s, d).off,
-                                    inv_range(s, d).n, 0, d > 0, 0, stream_)));
+            ECK((launch_sweep<B>(s, d, inv_variant[s][d], 0, 0, stream_)));
         for (int c = 0; c < kLineSchemes; ++c)
             ECK((launch_crweno<B>(kLineScheme[c], d, d_boxes_, it + r_cr_[c][d].off,
                                   r_cr_[c][d].n, 0, d > 0, cr_nmax_[c][d], cr_ms_[c][d], 0,

@@ -77,6 +77,14 @@ public:
                                     {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1},
                                     {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}};
     double inv_tune_ms[kSchemes][3][kInvVariants] = {};
+    // faces per thread and cells per tile of variant v (marched pairs: both are
+    // the chunk length)
+    int sweep_run(int s, int d, int v) const {
+        return marched(s, d, precision_ == NUC3D_MIXED) ? kMarchLen[v] : kInvRunLen[v];
+    }
+    int sweep_tile(int s, int d, int v) const {
+        return marched(s, d, precision_ == NUC3D_MIXED) ? kMarchLen[v] : kInvTileCells[v];
+    }
     // autotuned pencil depth of the 2.5-D stencil kernels: index into
     // kPencilDepths (-1: not tuned yet), the measured milliseconds of one
     // viscous-flux + update pass per depth, and the active cells it was tuned
@@ -128,10 +136,14 @@ private:
     };
     Range r_prim_;
     Range r_inv_[kSchemes][3][kInvTileClasses];  // [scheme id][dir][32/64-cell tiles]
-    // the work list of the variant the autotuner chose (32-cell tiles before)
-    const Range &inv_range(int s, int d) const {
-        return r_inv_[s][d][inv_variant[s][d] < 0 ? 0 : inv_tile_class(inv_variant[s][d])];
-    }
+    // marched pairs (marched()): one list of line groups whatever the chunk
+    // length, and the longest line of each launch
+    Range r_march_[kSchemes][3];
+    int march_nmax_[kSchemes][3] = {};
+    bool has_sweep(int s, int d) const { return r_inv_[s][d][0].n > 0 || r_march_[s][d].n > 0; }
+    // variant v of the directional sweep of scheme s on this batch's boxes
+    template <typename B>
+    cudaError_t launch_sweep(int s, int d, int v, int in, int prim_mode, cudaStream_t st);
     // 2.5-D stencil tiles per [stencil class (kVisReach)][pencil depth of
     // kPencilDepths]
     Range r_25d_[kVisClasses][3];

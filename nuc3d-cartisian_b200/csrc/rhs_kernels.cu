@@ -762,15 +762,14 @@ cudaError_t launch_inviscid(int scheme, int dir, int variant, const BoxDev *boxe
                             const WorkItem *items, int nitems, int in_slot, int accumulate,
                             int prim_mode, cudaStream_t st) {
     if (nitems <= 0) return cudaSuccess;
-    if (scheme == SCHEME_JS) {
-        if (dir == 0) return launch_v<SCHEME_JS, 0, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
-        if (dir == 1) return launch_v<SCHEME_JS, 1, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
-        return launch_v<SCHEME_JS, 2, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
-    }
-    if (scheme == SCHEME_Z) {
-        if (dir == 0) return launch_v<SCHEME_Z, 0, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
-        if (dir == 1) return launch_v<SCHEME_Z, 1, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
-        return launch_v<SCHEME_Z, 2, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+    // (JS and Z along y and z: FP32 only, FP64 marches, see marched())
+    if (scheme == SCHEME_JS && dir == 0) return launch_v<SCHEME_JS, 0, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+    if (scheme == SCHEME_Z && dir == 0) return launch_v<SCHEME_Z, 0, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+    if constexpr (sizeof(B) == 4) {
+        if (scheme == SCHEME_JS && dir == 1) return launch_v<SCHEME_JS, 1, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+        if (scheme == SCHEME_JS) return launch_v<SCHEME_JS, 2, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+        if (scheme == SCHEME_Z && dir == 1) return launch_v<SCHEME_Z, 1, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+        if (scheme == SCHEME_Z) return launch_v<SCHEME_Z, 2, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
     }
     if (scheme == SCHEME_W7) {
         if (dir == 0) return launch_v<SCHEME_W7, 0, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
@@ -803,12 +802,15 @@ static cudaError_t prepare_t() {
 }
 template <int SCHEME, int DIR, typename B>
 static cudaError_t prepare_runs() {
+    if constexpr (marched(SCHEME, DIR, sizeof(B) == 4)) return cudaSuccess;
+    else {
     cudaError_t e[kInvVariants] = {prepare_t<SCHEME, DIR, B, 1, 32>(), prepare_t<SCHEME, DIR, B, 2, 32>(),
                                    prepare_t<SCHEME, DIR, B, 4, 32>(), prepare_t<SCHEME, DIR, B, 2, 64>(),
                                    prepare_t<SCHEME, DIR, B, 4, 64>()};
     for (cudaError_t x : e)
         if (x != cudaSuccess) return x;
     return cudaSuccess;
+    }
 }
 template <typename B>
 static cudaError_t prepare_all() {

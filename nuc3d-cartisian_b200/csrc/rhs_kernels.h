@@ -138,6 +138,20 @@ template <typename B>
 cudaError_t launch_inviscid(int scheme, int dir, int variant, const BoxDev *boxes,
                             const WorkItem *items, int nitems, int in_slot, int accumulate,
                             int prim_mode, cudaStream_t st);
+// Marching y and z sweeps (march_kernels.cu) of the FP64 WENO5-JS / WENO5-Z
+// pairs: a work item is (box, group of 32 lines), the launch walks each line
+// in chunks of `len` cells (nmax: the longest line among the launch's boxes)
+// and adds to the RHS accumulator.  The autotuner's variant v of such a pair
+// is the chunk length kMarchLen[v]: short chunks give small boxes enough
+// teams, long ones re-read less of the chunk's 6-cell overlap (256^3 z: 8 to
+// 128 cells 0.95, 0.78, 0.67, 0.60, 0.57 ms; 97 x 61 x 45: 22, 20, 22, 26, 26 us).
+constexpr int kMarchLen[kInvVariants] = {8, 16, 32, 64, 128};
+constexpr bool marched(int scheme, int dir, bool mixed) {
+    return !mixed && dir > 0 && (scheme == SCHEME_JS || scheme == SCHEME_Z);
+}
+cudaError_t prepare_march_kernels();
+cudaError_t launch_march(int scheme, int dir, const BoxDev *boxes, const WorkItem *items,
+                         int nitems, int nmax, int in_slot, int len, cudaStream_t st);
 // raises the dynamic shared-memory limits of the 2.5-D stencil kernels
 cudaError_t prepare_stencil_kernels(bool mixed);
 // Stencil classes of the 2.5-D kernels: boxes whose three directions use cd6
