@@ -440,13 +440,14 @@ int Engine::rebuild() {
     ECK(cudaStreamSynchronize(stream_));
     const bool mixed = precision_ == NUC3D_MIXED;
     std::vector<BoxDev> table(boxes_.size());
-    std::vector<WorkItem> prim, st25[kVisClasses][3], inv[kSchemes][3][kInvTileClasses],
+    std::vector<WorkItem> prim, st25[kVisClasses], inv[kSchemes][3][kInvTileClasses],
         march[kSchemes][3], cr[kLineSchemes][3];
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d) march_nmax_[s][d] = 0;
     const int crtl = crweno_tile_lines();
     for (int c = 0; c < kLineSchemes; ++c)
         for (int d = 0; d < 3; ++d) cr_nmax_[c][d] = cr_ms_[c][d] = 0;
+    for (int c = 0; c < kVisClasses; ++c) nzmax_[c] = 0;
     any_visc_ = false;
     nactive_ = 0;
     active_cells_ = 0;
@@ -465,11 +466,9 @@ int Engine::rebuild() {
             prim.push_back({id, (int)c, (int)std::min<long long>(kPrimChunk, p.N - c * kPrimChunk), 0});
         boxes_[i].prim_n = (int)prim.size() - boxes_[i].prim_off;
         const int vc = vis_class(p);
-        for (int v = 0; v < 3; ++v)
-            for (int z = 0; z < ceil_div(p.n[2], kPencilDepths[v]); ++z)
-                for (int y = 0; y < ceil_div(p.n[1], kT25Y); ++y)
-                    for (int x = 0; x < ceil_div(p.n[0], kT25X); ++x)
-                        st25[vc][v].push_back({id, x, y, z});
+        nzmax_[vc] = std::max(nzmax_[vc], p.n[2]);
+        for (int y = 0; y < ceil_div(p.n[1], kT25Y); ++y)
+            for (int x = 0; x < ceil_div(p.n[0], kT25X); ++x) st25[vc].push_back({id, x, y, 0});
         for (int d = 0; d < 3; ++d) {
             int s = p.scheme[d];
             if (line_slot(s) >= 0) {
@@ -522,8 +521,7 @@ int Engine::rebuild() {
         all.insert(all.end(), v.begin(), v.end());
     };
     append(prim, r_prim_);
-    for (int c = 0; c < kVisClasses; ++c)
-        for (int v = 0; v < 3; ++v) append(st25[c][v], r_25d_[c][v]);
+    for (int c = 0; c < kVisClasses; ++c) append(st25[c], r_25d_[c]);
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d)
             for (int tc = 0; tc < kInvTileClasses; ++tc) append(inv[s][d][tc], r_inv_[s][d][tc]);
@@ -556,7 +554,7 @@ int Engine::rebuild() {
     ECK(prepare_stencil_kernels(mixed));
     int per_stage = 0;
     for (int c = 0; c < kVisClasses; ++c)
-        per_stage += (any_visc_ && r_25d_[c][0].n > 0) + (r_25d_[c][0].n > 0);
+        per_stage += (any_visc_ && r_25d_[c].n > 0) + (r_25d_[c].n > 0);
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d) per_stage += has_sweep(s, d);
     for (int c = 0; c < kLineSchemes; ++c)
@@ -683,9 +681,9 @@ cudaError_t Engine::launch_sweep(int s, int d, int v, int in, int prim_mode, cud
 template <typename B>
 cudaError_t Engine::launch_visc_classes(int v, cudaStream_t st) {
     for (int c = 0; c < kVisClasses; ++c) {
-        const Range &rg = r_25d_[c][v];
-        cudaError_t e = launch_visc_flux<B>(d_boxes_, d_items_ + rg.off, rg.n, kPencilDepths[v],
-                                            kVisReach[c], st);
+        const Range &rg = r_25d_[c];
+        cudaError_t e = launch_visc_flux<B>(d_boxes_, d_items_ + rg.off, rg.n, nzmax_[c],
+                                            kPencilDepths[v], kVisReach[c], st);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -694,9 +692,9 @@ cudaError_t Engine::launch_visc_classes(int v, cudaStream_t st) {
 template <typename B>
 cudaError_t Engine::launch_update_classes(int v, StageArgs sa, cudaStream_t st) {
     for (int c = 0; c < kVisClasses; ++c) {
-        const Range &rg = r_25d_[c][v];
-        cudaError_t e = launch_update<B>(d_boxes_, d_items_ + rg.off, rg.n, kPencilDepths[v], sa,
-                                         any_visc_, kVisReach[c], st);
+        const Range &rg = r_25d_[c];
+        cudaError_t e = launch_update<B>(d_boxes_, d_items_ + rg.off, rg.n, nzmax_[c],
+                                         kPencilDepths[v], sa, any_visc_, kVisReach[c], st);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -733,19 +731,26 @@ int Engine::enqueue_step(cudaStream_t s) {
 // update is timed as a first stage, which writes only the u1 slot that the
 // next step's first stage overwrites (and no residual), so timing on the
 // live state changes nothing.
+long long Engine::pencil_blocks(int v) const {
+    long long b = 0;
+    for (int c = 0; c < kVisClasses; ++c)
+        b += (long long)r_25d_[c].n * ceil_div(nzmax_[c], kPencilDepths[v]);
+    return b;
+}
+
 int Engine::autotune() {
     bool need_sweep = false;
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d)
             need_sweep = need_sweep || (has_sweep(s, d) && inv_variant[s][d] < 0);
     const bool need_pencil =
-        (r_25d_[0][0].n > 0 || r_25d_[1][0].n > 0) &&
+        (r_25d_[0].n > 0 || r_25d_[1].n > 0) &&
         (pencil_variant < 0 || 2 * active_cells_ < pencil_tuned_cells ||
                             active_cells_ > 2 * pencil_tuned_cells);
     if (!need_sweep && !need_pencil) return NUC3D_OK;
     // NUC3D_SWEEP_RUN=1|2|4 pins the run length (32-cell tiles; with
     // NUC3D_SWEEP_TILE=64, runs of 2 or 4 on 64-cell tiles) and
-    // NUC3D_PENCIL_DEPTH=16|32|64 the pencil depth (reproducibility studies)
+    // NUC3D_PENCIL_DEPTH=2|4|8|16|32|64 the pencil depth (reproducibility studies)
     if (need_sweep) {
         if (const char *pin = std::getenv("NUC3D_SWEEP_RUN")) {
             const int run = std::atoi(pin);
@@ -767,7 +772,7 @@ int Engine::autotune() {
         if (const char *pin = std::getenv("NUC3D_PENCIL_DEPTH")) {
             const int want = std::atoi(pin);
             pencil_variant = 0;
-            for (int v = 0; v < 3; ++v)
+            for (int v = 0; v < kPencils; ++v)
                 if (kPencilDepths[v] == want) pencil_variant = v;
             pencil_tuned_cells = active_cells_;
             tune_pencil = false;
@@ -822,7 +827,14 @@ int Engine::autotune() {
         }
     if (tune_pencil && rc == NUC3D_OK) {
         int best = 0;
-        for (int v = 0; v < 3 && rc == NUC3D_OK; ++v) {
+        for (int v = 0; v < kPencils && rc == NUC3D_OK; ++v) {
+            // a short depth only where depth 16 makes few blocks and the
+            // next longer depth was the best so far
+            const int longer = v == 3 ? 1 : v - 1;
+            if (v > 2 && (pencil_blocks(1) > kPencilShortBlocks || best != longer)) {
+                pencil_tune_ms[v] = 0.0;
+                continue;
+            }
             const StageArgs sa{0, 0, 1, nullptr};
             const double ms = time3([&]() {
                 cudaError_t err = cudaSuccess;

@@ -90,7 +90,7 @@ public:
     // viscous-flux + update pass per depth, and the active cells it was tuned
     // at (a batch that grows or shrinks past 2x is tuned again)
     int pencil_variant = -1;
-    double pencil_tune_ms[3] = {};
+    double pencil_tune_ms[kPencils] = {};
     long long pencil_tuned_cells = 0;
 
     static long long box_bytes(const nuc3d_box_desc &d);
@@ -144,10 +144,15 @@ private:
     // variant v of the directional sweep of scheme s on this batch's boxes
     template <typename B>
     cudaError_t launch_sweep(int s, int d, int v, int in, int prim_mode, cudaStream_t st);
-    // 2.5-D stencil tiles per [stencil class (kVisReach)][pencil depth of
-    // kPencilDepths]
-    Range r_25d_[kVisClasses][3];
+    // 2.5-D stencil tiles per stencil class (kVisReach), and the most planes
+    // among its boxes
+    Range r_25d_[kVisClasses];
+    int nzmax_[kVisClasses] = {};
     long long active_cells_ = 0;
+    long long pencil_blocks(int v) const;  // blocks of a 2.5-D launch at depth v
+    // blocks up to which the short pencils are worth timing: two waves of 148
+    // SMs x 2 blocks at depth 16
+    static constexpr long long kPencilShortBlocks = 600;
     int pv() const { return pencil_variant < 0 ? 0 : pencil_variant; }
     // Mixed precision stages each line's split fluxes as FP32 offsets from
     // their value at the tile's first cell, so the rounding depends on where
