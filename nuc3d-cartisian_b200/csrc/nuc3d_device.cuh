@@ -964,24 +964,44 @@ __device__ __forceinline__ B cd6(B m3, B m2, B m1, B p1, B p2, B p3, B inv_dx) {
     return (B(K::CD3) * (p3 - m3) + B(K::CD2) * (p2 - m2) + B(K::CD1) * (p1 - m1)) * inv_dx;
 }
 
-// Derivative of a whole-box field f at cell (i, j, k) along axis d with the
-// periodic wrap by the direction's differential scheme (centraldifference6th
-// .cpp:44-46, centraldifference2nd.cpp:44, centraldifference8th.cpp:120-123
-// on one rank), FP64; the diagnostics' gradients (statistics, spectra).
-__device__ __forceinline__ double diff_at(const double *f, const BoxParams &p, int i, int j, int k,
-                                          int d) {
-    const int n = p.n[d];
-    const int c = d == 0 ? i : (d == 1 ? j : k);
-    const long long base = (long long)i + p.stride[1] * j + p.stride[2] * k - p.stride[d] * c;
-    auto at = [&](int o) { return f[base + p.stride[d] * wrap(c + o, n)]; };
-    if (p.vis[d] == VIS_CD2) return K::C21 * (at(1) - at(-1)) / p.d[d];
-    if (p.vis[d] == VIS_CD8)
-        return (K::C84 * (at(4) - at(-4)) + K::C83 * (at(3) - at(-3)) +
-                K::C82 * (at(2) - at(-2)) + K::C81 * (at(1) - at(-1))) /
-               p.d[d];
-    return (K::CD3 * (at(3) - at(-3)) + K::CD2 * (at(2) - at(-2)) + K::CD1 * (at(1) - at(-1))) /
-           p.d[d];
+// Derivatives of whole-box fields at one cell with the periodic wrap by the
+// directions' differential schemes (centraldifference6th.cpp:44-46,
+// centraldifference2nd.cpp:44, centraldifference8th.cpp:120-123 on one rank),
+// FP64; the diagnostics' gradients (statistics, spectra).  R: 3 where every
+// direction uses cd6, else 4 (the scheme as its coefficients of
+// f(i+m) - f(i-m)).  The neighbours' indices are formed once per cell and
+// shared by the fields (a box holds at most 2^31 cells).
+__host__ __device__ __forceinline__ int diff_reach(const BoxParams &p) {
+    return p.vis[0] == VIS_CD6 && p.vis[1] == VIS_CD6 && p.vis[2] == VIS_CD6 ? 3 : 4;
 }
+template <int R>
+struct DiffAt {
+    unsigned o[3][2 * R];  // [axis][cells -R..-1, 1..R]
+    __device__ __forceinline__ DiffAt(const BoxParams &p, unsigned c) {
+        const unsigned nx = p.n[0], ny = p.n[1];
+        const unsigned line = c / nx, i = c - line * nx, k = line / ny, j = line - k * ny;
+        const int x[3] = {(int)i, (int)j, (int)k};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int n = p.n[d], st = (int)p.stride[d];
+#pragma unroll
+            for (int m = 1; m <= R; ++m) {
+                o[d][R - m] = c + (x[d] >= m ? -m : n - m) * st;
+                o[d][R + m - 1] = c + (x[d] + m < n ? m : m - n) * st;
+            }
+        }
+    }
+    __device__ __forceinline__ double operator()(const double *f, const BoxParams &p, int d) const {
+        double r = 0.0;
+#pragma unroll
+        for (int m = R; m >= 1; --m) {
+            const double df = f[o[d][R + m - 1]] - f[o[d][R - m]];
+            const double c = R == 4 ? p.vcoef[d][m - 1] : (m == 1 ? K::CD1 : (m == 2 ? K::CD2 : K::CD3));
+            r = fma_(c, df, r);
+        }
+        return r * p.inv_d[d];
+    }
+};
 
 // Viscosity and heat-conduction coefficient (physicsModel.cpp:193-266).
 template <typename B>

@@ -4,11 +4,16 @@
 //
 //   k_spec_fields  u, v, w, the helicity field w.u, the enstrophy field
 //                  |w|^2/2 (solveQ's fields, postproc.cpp:812-853, vorticity
-//                  from the differential scheme's gradients), density and pressure, as complex
-//                  fields with zero imaginary part;
-//   cuFFT          one batched forward 3-D Z2Z transform of the seven fields
-//                  (FFTW_FORWARD sign; the 1/N of fft.cpp:277-278 is applied
-//                  when binning);
+//                  from the differential scheme's gradients), density and
+//                  pressure, rows padded to 2 (nx/2 + 1) reals;
+//   cuFFT          one batched forward 3-D D2Z transform of the seven fields in
+//                  place (FFTW_FORWARD sign; the 1/N of fft.cpp:277-278 is
+//                  applied when binning).  The fields are real, so the modes
+//                  with kx < 0 are the conjugates of their mirrors and carry
+//                  the same energies: half the transform, scratch and binning
+//                  of complex fields with a zero imaginary part.  (A mode on
+//                  a Nyquist plane, whose mirror the fold takes to the same
+//                  sign, has |k| >= kmax and is in no shell.);
 //   k_spec_bin     per mode: the folded wavenumber, the compressive /
 //                  solenoidal / helical split of the velocity transform
 //                  (postproc.cpp:1013-1101) and the shell of each binning.
@@ -16,9 +21,14 @@
 //                  substituted at k = 0 (fft.cpp:424-435, the mean flow lands
 //                  in shell 1); the scalar spectra use the unfolded
 //                  i^2 + j^2 + k^2 of fft.cpp:517-531 (only the non-negative
-//                  octant is counted).  Each block adds its modes into shared
-//                  shell sums in a fixed order;
-//   k_spec_reduce  adds the blocks' shell sums in a fixed order.
+//                  octant is counted).  A warp takes 32 modes of a (j, k) row
+//                  at a time; along a row the shells do not decrease, so a
+//                  segmented warp scan sums each shell's run and the runs'
+//                  last lanes add to the warp's own shell sums in shared
+//                  memory, each shell once: a fixed order without atomics
+//                  (128^3: 502 us with one thread per spectrum adding a
+//                  block's modes one by one);
+//   k_spec_reduce  adds the blocks' shell sums in a fixed order, a warp per sum.
 // The grid is fixed, so a box gives the same bits alone or in any batch.
 #include <cufft.h>
 
@@ -31,28 +41,29 @@ namespace {
 
 constexpr int kThreads = 256;
 
-__global__ void __launch_bounds__(kThreads) k_spec_fields(BoxDev b, double2 *F) {
+template <int R>
+__global__ void __launch_bounds__(kThreads) k_spec_fields(BoxDev b, double *F) {
     const BoxParams &p = b.p;
-    const long long N = p.N;
     const double *rho = fieldU(b, 0, 0);
     const double *u = fieldW(b, 0), *v = fieldW(b, 1), *w = fieldW(b, 2), *pr = fieldW(b, 3);
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < N;
-         c += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(c % p.n[0]);
-        const int j = (int)((c / p.n[0]) % p.n[1]);
-        const int k = (int)(c / ((long long)p.n[0] * p.n[1]));
+    const unsigned nx = p.n[0];
+    const unsigned pad = 2 * (nx / 2 + 1) - nx;
+    const long long NF = p.N + (long long)pad * (p.N / nx);
+    for (long long cc = blockIdx.x * (long long)blockDim.x + threadIdx.x; cc < p.N;
+         cc += (long long)gridDim.x * blockDim.x) {
+        const unsigned c = (unsigned)cc;
+        const DiffAt<R> at(p, c);
         const double u0 = u[c], u1 = v[c], u2 = w[c];
-        const double uy = diff_at(u, p, i, j, k, 1), uz = diff_at(u, p, i, j, k, 2);
-        const double vx = diff_at(v, p, i, j, k, 0), vz = diff_at(v, p, i, j, k, 2);
-        const double wx = diff_at(w, p, i, j, k, 0), wy = diff_at(w, p, i, j, k, 1);
-        const double w0 = wy - vz, w1 = uz - wx, w2 = vx - uy;
-        F[c] = make_double2(u0, 0.0);
-        F[N + c] = make_double2(u1, 0.0);
-        F[2 * N + c] = make_double2(u2, 0.0);
-        F[3 * N + c] = make_double2(w0 * u0 + w1 * u1 + w2 * u2, 0.0);
-        F[4 * N + c] = make_double2((w0 * w0 + w1 * w1 + w2 * w2) * 0.5, 0.0);
-        F[5 * N + c] = make_double2(rho[c], 0.0);
-        F[6 * N + c] = make_double2(pr[c], 0.0);
+        const double w0 = at(w, p, 1) - at(v, p, 2), w1 = at(u, p, 2) - at(w, p, 0),
+                     w2 = at(v, p, 0) - at(u, p, 1);
+        double *const o = F + cc + (long long)pad * (c / nx);
+        o[0] = u0;
+        o[NF] = u1;
+        o[2 * NF] = u2;
+        o[3 * NF] = w0 * u0 + w1 * u1 + w2 * u2;
+        o[4 * NF] = (w0 * w0 + w1 * w1 + w2 * w2) * 0.5;
+        o[5 * NF] = rho[c];
+        o[6 * NF] = pr[c];
     }
 }
 
@@ -63,114 +74,134 @@ __device__ __forceinline__ int shell_of(double kmag) {
 }
 
 __device__ __forceinline__ double folded(int i, int n) {
-    return (i >= n / 2.0) ? (double)i - n : (double)i;  // fft.cpp:424-426
+    return (2 * i >= n) ? (double)i - n : (double)i;  // fft.cpp:424-426
 }
 
 __device__ __forceinline__ double sq(double x) { return x * x; }
 
+// adds the lanes' values to h[q * ks + shell] (shell < 0: nowhere); equal
+// shells sit in adjacent lanes
+template <int NQ>
+__device__ __forceinline__ void add_runs(double (&v)[NQ], int shell, double *h, int ks) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const bool same = __shfl_up_sync(0xffffffffu, shell, o) == shell && lane >= o;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const double t = __shfl_up_sync(0xffffffffu, v[q], o);
+            if (same) v[q] += t;
+        }
+    }
+    const int next = __shfl_down_sync(0xffffffffu, shell, 1);
+    if (shell >= 0 && (lane == 31 || next != shell)) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) h[q * ks + shell] += v[q];
+    }
+    __syncwarp();
+}
+
 __global__ void __launch_bounds__(kThreads) k_spec_bin(const double2 *F, int nx, int ny, int nz,
                                                         int kmax, double *partials) {
-    extern __shared__ __align__(16) double sm[];
-    const int ks = kmax + 1;
-    double *hist = sm;                        // [kSpectra][kmax + 1]
-    double *val = hist + kSpectra * ks;       // [kSpectra][kThreads]
-    int *shell = reinterpret_cast<int *>(val + kSpectra * kThreads);  // [2][kThreads]
-    for (int t = threadIdx.x; t < kSpectra * ks; t += blockDim.x) hist[t] = 0.0;
-    const long long N = (long long)nx * ny * nz;
-    const long long chunk = (N + gridDim.x - 1) / gridDim.x;
-    const long long m0 = blockIdx.x * chunk;
-    const long long m1 = m0 + chunk < N ? m0 + chunk : N;
-    const double dN = (double)N;
+    extern __shared__ __align__(16) double sm[];  // [warp][kSpectra][kmax + 1]
+    const int NW = blockDim.x >> 5, ks = kmax + 1, nh = nx / 2 + 1;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int t = threadIdx.x; t < NW * kSpectra * ks; t += blockDim.x) sm[t] = 0.0;
     __syncthreads();
-    for (long long base = m0; base < m1; base += kThreads) {
-        const long long m = base + threadIdx.x;
-        int sk = -1, so = -1;
-        double v[kSpectra];
-#pragma unroll
-        for (int q = 0; q < kSpectra; ++q) v[q] = 0.0;
-        if (m < m1) {
-            const int i = (int)(m % nx), j = (int)((m / nx) % ny), k = (int)(m / ((long long)nx * ny));
-            const double kx = folded(i, nx), ky = folded(j, ny), kz = folded(k, nz);
-            double kmag = sqrt(kx * kx + ky * ky + kz * kz);
+    double *const hist = sm + warp * kSpectra * ks;
+    const long long rows = (long long)ny * nz, NH = rows * nh;
+    const double inv_n = 1.0 / ((double)nx * ny * nz), kc = (double)kmax;
+    for (long long row = blockIdx.x * NW + warp; row < rows; row += (long long)gridDim.x * NW) {
+        const int k = (int)(row / ny), j = (int)(row - (long long)k * ny);
+        const double ky = folded(j, ny), kz = folded(k, nz);
+        const double k2 = ky * ky + kz * kz;
+        const long long r2 = (long long)j * j + (long long)k * k;
+        const bool scal = r2 < (long long)kmax * kmax;  // (implies k2 < kmax^2)
+        if (k2 >= kc * kc) continue;
+        for (int i0 = 0; i0 < nh && i0 < kmax; i0 += 32) {
+            const int i = i0 + lane;
+            const long long m = row * nh + i;
+            double kmag = sqrt((double)i * i + k2);
             if (kmag < 1e-6) kmag = 1.0;
-            if (kmag < kmax) {
-                sk = shell_of(kmag);
+            const bool in = i < nh && kmag < kc;
+            double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+            if (in) {
+                const double ik = 1.0 / kmag;
+                // unit wavevector (the zero vector at k = 0)
+                const double e[3] = {folded(i, nx) * ik, ky * ik, kz * ik};
                 double ur[3], ui[3];
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
-                    const double2 f = F[d * N + m];
-                    ur[d] = f.x / dN;  // fft.cpp:277-278 (division, as normalization())
-                    ui[d] = f.y / dN;
+                    const double2 f = F[d * NH + m];
+                    ur[d] = f.x * inv_n;  // fft.cpp:277-278
+                    ui[d] = f.y * inv_n;
                 }
-                const double kv[3] = {kx, ky, kz};
-                const double ku_r = (kx * ur[0] + ky * ur[1] + kz * ur[2]) / kmag;
-                const double ku_i = (kx * ui[0] + ky * ui[1] + kz * ui[2]) / kmag;
-                double sr[3], si[3], cr[3], ci[3];
+                const double ku_r = e[0] * ur[0] + e[1] * ur[1] + e[2] * ur[2];
+                const double ku_i = e[0] * ui[0] + e[1] * ui[1] + e[2] * ui[2];
+                double sr[3], si[3];
+                double a = 0.0, c = 0.0, s = 0.0, l = 0.0, r = 0.0;
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
-                    sr[d] = ur[d] - ku_r * kv[d] / kmag;
-                    si[d] = ui[d] - ku_i * kv[d] / kmag;
-                    cr[d] = ur[d] - sr[d];
-                    ci[d] = ui[d] - si[d];
+                    sr[d] = ur[d] - ku_r * e[d];
+                    si[d] = ui[d] - ku_i * e[d];
+                    a += sq(ur[d]) + sq(ui[d]);
+                    c += sq(ur[d] - sr[d]) + sq(ui[d] - si[d]);
+                    s += sq(sr[d]) + sq(si[d]);
                 }
                 // i k x s / |k| (postproc.cpp:1052-1059)
-                const double xr[3] = {-(ky * si[2] - kz * si[1]) / kmag,
-                                      (kx * si[2] - kz * si[0]) / kmag,
-                                      -(kx * si[1] - ky * si[0]) / kmag};
-                const double xi[3] = {(ky * sr[2] - kz * sr[1]) / kmag,
-                                      -(kx * sr[2] - kz * sr[0]) / kmag,
-                                      (kx * sr[1] - ky * sr[0]) / kmag};
-                double e[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+                const double xr[3] = {-(e[1] * si[2] - e[2] * si[1]), e[0] * si[2] - e[2] * si[0],
+                                      -(e[0] * si[1] - e[1] * si[0])};
+                const double xi[3] = {e[1] * sr[2] - e[2] * sr[1], -(e[0] * sr[2] - e[2] * sr[0]),
+                                      e[0] * sr[1] - e[1] * sr[0]};
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
-                    e[0] += sq(ur[d]) + sq(ui[d]);
-                    e[1] += sq(cr[d]) + sq(ci[d]);
-                    e[2] += sq(sr[d]) + sq(si[d]);
-                    e[3] += sq(0.5 * (sr[d] - xr[d])) + sq(0.5 * (si[d] - xi[d]));
-                    e[4] += sq(0.5 * (sr[d] + xr[d])) + sq(0.5 * (si[d] + xi[d]));
+                    l += sq(sr[d] - xr[d]) + sq(si[d] - xi[d]);
+                    r += sq(sr[d] + xr[d]) + sq(si[d] + xi[d]);
                 }
-#pragma unroll
-                for (int q = 0; q < 5; ++q) v[q] = 0.5 * e[q];
+                // 1/2, twice where the mirror mode is left out
+                const double w = i == 0 ? 0.5 : 1.0;
+                v[0] = w * a;
+                v[1] = w * c;
+                v[2] = w * s;
+                v[3] = 0.25 * w * l;
+                v[4] = 0.25 * w * r;
             }
-            const long long k0 = (long long)i * i + (long long)j * j + (long long)k * k;
-            if (k0 < (long long)kmax * kmax) {
-                so = shell_of(sqrt((double)k0));
+            add_runs<5>(v, in ? shell_of(kmag) : -1, hist, ks);
+            if (!scal) continue;
+            const long long k0 = (long long)i * i + r2;
+            const bool on = i < nh && k0 < (long long)kmax * kmax;
+            double q[4] = {0.0, 0.0, 0.0, 0.0};
+            if (on) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const double2 f = F[(3 + q) * N + m];
-                    v[5 + q] = sq(f.x / dN) + sq(f.y / dN);
+                for (int d = 0; d < 4; ++d) {
+                    const double2 f = F[(3 + d) * NH + m];
+                    q[d] = sq(f.x * inv_n) + sq(f.y * inv_n);
                 }
             }
+            add_runs<4>(q, on ? shell_of(sqrt((double)k0)) : -1, hist + 5 * ks, ks);
         }
-#pragma unroll
-        for (int q = 0; q < kSpectra; ++q) val[q * kThreads + threadIdx.x] = v[q];
-        shell[threadIdx.x] = sk;
-        shell[kThreads + threadIdx.x] = so;
-        __syncthreads();
-        if (threadIdx.x < kSpectra) {  // one thread per spectrum, modes in order
-            const int q = threadIdx.x;
-            const int *sh = shell + (q < 5 ? 0 : kThreads);
-            double *h = hist + q * ks;
-            const double *vq = val + q * kThreads;
-            for (int t = 0; t < kThreads; ++t)
-                if (sh[t] >= 0) h[sh[t]] += vq[t];
-        }
-        __syncthreads();
     }
-    for (int t = threadIdx.x; t < kSpectra * kmax; t += blockDim.x)
-        partials[(size_t)blockIdx.x * kSpectra * kmax + t] = hist[(t / kmax) * ks + t % kmax];
+    __syncthreads();
+    for (int t = threadIdx.x; t < kSpectra * kmax; t += blockDim.x) {
+        const int h = (t / kmax) * ks + t % kmax;
+        double s = 0.0;
+        for (int w = 0; w < NW; ++w) s += sm[w * kSpectra * ks + h];
+        partials[(size_t)blockIdx.x * kSpectra * kmax + t] = s;
+    }
 }
 
+// one warp per sum
 __global__ void k_spec_reduce(const double *partials, int nblocks, int n, double *out) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (t >= n) return;
     double s = 0.0;
-    for (int b = 0; b < nblocks; ++b) s += partials[(size_t)b * n + t];
-    out[t] = s;
+    for (int b = lane; b < nblocks; b += 32) s += partials[(size_t)b * n + t];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) out[t] = s;
 }
 
 size_t fields_bytes(const BoxParams &p) {
-    return sizeof(double2) * kSpectraFields * (size_t)p.N;
+    return sizeof(double2) * kSpectraFields * (size_t)(p.n[0] / 2 + 1) * p.n[1] * p.n[2];
 }
 
 }  // namespace
@@ -184,24 +215,28 @@ cudaError_t launch_spectra(const BoxDev &b, void *scratch, double *d_out, int *f
                            cudaStream_t st) {
     const BoxParams &p = b.p;
     const int kmax = spectra_kmax(p);
-    double2 *F = static_cast<double2 *>(scratch);
+    double *F = static_cast<double *>(scratch);
     double *partials = reinterpret_cast<double *>(static_cast<char *>(scratch) + fields_bytes(p));
     *fft_status = CUFFT_SUCCESS;
-    k_spec_fields<<<4 * 148, kThreads, 0, st>>>(b, F);
+    if (diff_reach(p) == 3)
+        k_spec_fields<3><<<4 * 148, kThreads, 0, st>>>(b, F);
+    else
+        k_spec_fields<4><<<4 * 148, kThreads, 0, st>>>(b, F);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     // forward 3-D transforms of the seven fields (x fastest: dims nz, ny, nx)
     cufftHandle plan;
-    long long dims[3] = {p.n[2], p.n[1], p.n[0]};
+    const long long nh = p.n[0] / 2 + 1, rows = (long long)p.n[1] * p.n[2];
+    long long dims[3] = {p.n[2], p.n[1], p.n[0]}, real[3] = {p.n[2], p.n[1], 2 * nh},
+              half[3] = {p.n[2], p.n[1], nh};
     size_t work = 0;
     cufftResult r = cufftCreate(&plan);
     if (r == CUFFT_SUCCESS) {
-        r = cufftMakePlanMany64(plan, 3, dims, nullptr, 1, p.N, nullptr, 1, p.N, CUFFT_Z2Z,
-                                kSpectraFields, &work);
+        r = cufftMakePlanMany64(plan, 3, dims, real, 1, 2 * nh * rows, half, 1, nh * rows,
+                                CUFFT_D2Z, kSpectraFields, &work);
         if (r == CUFFT_SUCCESS) r = cufftSetStream(plan, st);
         if (r == CUFFT_SUCCESS)
-            r = cufftExecZ2Z(plan, reinterpret_cast<cufftDoubleComplex *>(F),
-                             reinterpret_cast<cufftDoubleComplex *>(F), CUFFT_FORWARD);
+            r = cufftExecD2Z(plan, F, reinterpret_cast<cufftDoubleComplex *>(F));
         e = cudaStreamSynchronize(st);  // the plan's work area outlives the transform
         cufftDestroy(plan);
     }
@@ -210,16 +245,20 @@ cudaError_t launch_spectra(const BoxDev &b, void *scratch, double *d_out, int *f
         return cudaErrorUnknown;
     }
     if (e != cudaSuccess) return e;
-    const size_t smem = sizeof(double) * (size_t)kSpectra * (kmax + 1 + kThreads) +
-                        sizeof(int) * 2 * kThreads;
+    // warps per block: as many shell tables as fit 200 KB, at most 8 (a box
+    // of 2^31 cells has kmax <= 645)
+    const size_t table = sizeof(double) * kSpectra * (size_t)(kmax + 1);
+    const int warps = (int)(200 * 1024 / table < 8 ? 200 * 1024 / table : 8);
+    const size_t smem = table * warps;
     if (smem > 48 * 1024) {
         e = cudaFuncSetAttribute(k_spec_bin, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem);
         if (e != cudaSuccess) return e;
     }
-    k_spec_bin<<<kSpecBlocks, kThreads, smem, st>>>(F, p.n[0], p.n[1], p.n[2], kmax, partials);
+    k_spec_bin<<<kSpecBlocks, 32 * warps, smem, st>>>(reinterpret_cast<const double2 *>(F), p.n[0],
+                                                    p.n[1], p.n[2], kmax, partials);
     const int n = kSpectra * kmax;
-    k_spec_reduce<<<(n + 127) / 128, 128, 0, st>>>(partials, kSpecBlocks, n, d_out);
+    k_spec_reduce<<<(n + 3) / 4, 128, 0, st>>>(partials, kSpecBlocks, n, d_out);
     return cudaGetLastError();
 }
 

@@ -9,13 +9,13 @@ namespace nuc3d {
 
 constexpr int kSpectra = 9;         // kin, kinc, kins, kinl, kinr, hel, ens, den, pre
 constexpr int kSpectraFields = 7;   // transformed fields: u, v, w, hel, ens, rho, p
-constexpr int kSpecBlocks = 592;    // fixed binning grid (4 x 148): results do not depend on the batch
+constexpr int kSpecBlocks = 296;    // fixed binning grid (2 x 148): results do not depend on the batch
 
 inline int spectra_kmax(const BoxParams &p) {
     int m = p.n[0] < p.n[1] ? p.n[0] : p.n[1];
     return (m < p.n[2] ? m : p.n[2]) / 2;
 }
-// device scratch of a spectra evaluation: the seven complex fields, the
+// device scratch of a spectra evaluation: the seven transformed fields, the
 // per-block shell partials and the result
 size_t spectra_scratch_bytes(const BoxParams &p);
 // Spectra of box b (W must hold the primitives of U[0]) into

@@ -35,27 +35,26 @@ __device__ void block_sum(double (&v)[NV], double *out) {
     }
 }
 
+// Bound by its 54 gradient loads per cell, which hit L1 / L2.
+template <int R>
 __global__ void __launch_bounds__(kThreads) k_stats(BoxDev b, double *partials) {
     const BoxParams &p = b.p;
     const double *rho = fieldU(b, 0, 0);
     const double *u = fieldW(b, 0), *v = fieldW(b, 1), *w = fieldW(b, 2);
     const double *cs = fieldW(b, 4), *T = fieldW(b, 5);
     const double s_nd = p.tref_nd;
+    const ViscConst<double> vc(p);
     double acc[kStatsSums];
 #pragma unroll
     for (int s = 0; s < kStatsSums; ++s) acc[s] = 0.0;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < p.N;
-         c += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(c % p.n[0]);
-        const int j = (int)((c / p.n[0]) % p.n[1]);
-        const int k = (int)(c / ((long long)p.n[0] * p.n[1]));
+    for (long long cc = blockIdx.x * (long long)blockDim.x + threadIdx.x; cc < p.N;
+         cc += (long long)gridDim.x * blockDim.x) {
+        const unsigned c = (unsigned)cc;
+        const DiffAt<R> at(p, c);
         const double u0 = u[c], u1 = v[c], u2 = w[c];
-        const double ux = diff_at(u, p, i, j, k, 0), uy = diff_at(u, p, i, j, k, 1),
-                     uz = diff_at(u, p, i, j, k, 2);
-        const double vx = diff_at(v, p, i, j, k, 0), vy = diff_at(v, p, i, j, k, 1),
-                     vz = diff_at(v, p, i, j, k, 2);
-        const double wx = diff_at(w, p, i, j, k, 0), wy = diff_at(w, p, i, j, k, 1),
-                     wz = diff_at(w, p, i, j, k, 2);
+        const double ux = at(u, p, 0), uy = at(u, p, 1), uz = at(u, p, 2);
+        const double vx = at(v, p, 0), vy = at(v, p, 1), vz = at(v, p, 2);
+        const double wx = at(w, p, 0), wy = at(w, p, 1), wz = at(w, p, 2);
         // postproc.cpp:812-853
         const double w0 = wy - vz, w1 = uz - wx, w2 = vx - uy;
         const double q0 = ux * vy + ux * wz + vy * wz - uy * vx - uz * wx - vz * wy;
@@ -78,13 +77,13 @@ __global__ void __launch_bounds__(kThreads) k_stats(BoxDev b, double *partials) 
         acc[15] += 0.5 * rho[c] * (u0 * u0 + u1 * u1 + u2 * u2);
         acc[16] += (u0 * u0 + u1 * u1 + u2 * u2) / 3.0;
         acc[17] += (ux * ux + vy * vy + wz * wz) / 3.0;
-        acc[18] += (pow(ux, 3.0) + pow(vy, 3.0) + pow(wz, 3.0)) / 3.0;
+        acc[18] += (ux * ux * ux + vy * vy * vy + wz * wz * wz) / 3.0;
         acc[19] += cs[c];
         const double Tc = T[c];
-        acc[20] += (1.0 + s_nd) / (Tc + s_nd) * pow(Tc, 1.5);
+        acc[20] += (1.0 + s_nd) / (Tc + s_nd) * (Tc * sqrt(Tc));
         acc[21] += rho[c];
         double miu, coeff;
-        viscosity<double>(p, Tc, miu, coeff);
+        vc.eval(Tc, miu, coeff);
         const double th = ux + vy + wz;
         acc[22] += miu * (om2 + 4.0 / 3.0 * th * th);
     }
@@ -104,7 +103,10 @@ __global__ void __launch_bounds__(kThreads) k_stats_reduce(const double *partial
 }  // namespace
 
 cudaError_t launch_stats(const BoxDev &b, double *scratch, cudaStream_t st) {
-    k_stats<<<kStatsBlocks, kThreads, 0, st>>>(b, scratch + kStatsSums);
+    if (diff_reach(b.p) == 3)
+        k_stats<3><<<kStatsBlocks, kThreads, 0, st>>>(b, scratch + kStatsSums);
+    else
+        k_stats<4><<<kStatsBlocks, kThreads, 0, st>>>(b, scratch + kStatsSums);
     k_stats_reduce<<<1, kThreads, 0, st>>>(scratch + kStatsSums, kStatsBlocks, scratch);
     return cudaGetLastError();
 }
