@@ -31,6 +31,7 @@
 #include <type_traits>
 
 #include "nuc3d_device.cuh"
+#include "op_kernels.h"
 #include "prim_device.cuh"
 #include "rhs_kernels.h"
 
@@ -143,6 +144,224 @@ size_t crweno_smem_bytes(int sch, int nmax, int ms, bool mixed) {
 
 int crweno_tile_lines() { return kCrTL; }
 
+// One warp's (line, sign) system: myF holds the line's split flux of sign sg (0:
+// '+', 1: '-'; warp-uniform), cell c at [c + H], and receives its face values,
+// face m at [m].  wA: the warp's rows [3][ms][32]; n cells, N unknowns, P lanes.
+template <typename B, int SCH>
+__device__ __forceinline__ void line_solve(B *const myF, B *const wA, int ms, int n, int N, int P,
+                                           bool bounded, int sg, int lane) {
+    constexpr int H = scheme_halo(SCH);
+    B *const wC = wA + ms * 32;
+    B *const wD = wC + ms * 32;
+    const int hl = lane;
+    // explicit faces of the bounded system: 0..H-1 and n-H+1..n
+    int xm = -1;
+    B xv = B(0);
+    // segment of this lane: rows r0 .. r1 (at least 2)
+    const bool act = hl < P;
+    const int r0 = act ? (hl * N) / P : 0;
+    const int r1 = act ? ((hl + 1) * N) / P - 1 : 1;
+    const int L = r1 - r0 + 1;
+    B fa = B(0), fc = B(0), fd = B(0);  // reduced unit-diagonal row of x_first
+    B la = B(0), lc = B(0), ld = B(0);  // reduced unit-diagonal row of x_last
+    // the row work of one sign; the sign (warp-uniform) is a compile-time
+    // constant inside, so each warp runs code without sign selects
+    auto segment = [&](auto sign) {
+        constexpr int S = decltype(sign)::value;
+        auto F = [&](int c) -> B { return myF[c + H]; };
+        // the sign (warp-uniform) only selects which cells feed a
+        // stencil ('+' reads upwind from the left, '-' from the right)
+        constexpr int dir = S == 0 ? 1 : -1;
+        // explicit face m: WENO5-JS (crweno5.cpp:425-837), hccs's WENO7
+        // (hccs.cpp:538-980) or hccs77's WENO7-Z (hccs77.cpp:330-818)
+        auto js = [&](int m) -> B {
+            if (SCH == SCHEME_HC || SCH == SCHEME_H77) {
+                const int c0 = S == 0 ? m - 4 : m + 3;
+                if (SCH == SCHEME_HC)
+                    return weno7_face_hc(F(c0), F(c0 + dir), F(c0 + 2 * dir),
+                                         F(c0 + 3 * dir), F(c0 + 4 * dir), F(c0 + 5 * dir),
+                                         F(c0 + 6 * dir));
+                return weno7_face(F(c0), F(c0 + dir), F(c0 + 2 * dir), F(c0 + 3 * dir),
+                                  F(c0 + 4 * dir), F(c0 + 5 * dir), F(c0 + 6 * dir));
+            }
+            const int c0 = S == 0 ? m - 3 : m + 2;
+            return weno5js_face(F(c0), F(c0 + dir), F(c0 + 2 * dir), F(c0 + 3 * dir),
+                                F(c0 + 4 * dir));
+        };
+        // lanes 0..2H-1: the explicit faces; lanes 2H and 2H+1: the
+        // identity rows' values (faces H and n-H), passed to the lanes
+        // that own those rows, so the warp evaluates explicit faces once
+        B did0 = B(0), did1 = B(0);
+        if (bounded) {
+            B v = B(0);
+            if (hl < 2 * H + 2) {
+                const int m = hl < H ? hl
+                                     : (hl < 2 * H ? n - 2 * H + 1 + hl
+                                                   : (hl == 2 * H ? H : n - H));
+                v = js(m);
+                if (hl < 2 * H) {
+                    xm = m;
+                    xv = v;
+                }
+            }
+            did0 = shfl(v, 2 * H);
+            did1 = shfl(v, 2 * H + 1);
+        }
+        if (act) {
+            // window w[k] = F(i - WO + k) of the current row's cell i (face
+            // i + 1): cells i-2..i+3 for the 5-cell rows, i-3..i+4 for
+            // hccs77's 7-cell rows
+            constexpr int WN = SCH == SCHEME_H77 ? 8 : 6, WO = SCH == SCHEME_H77 ? 3 : 2;
+            int i = bounded ? r0 + H - 1 : r0 - 1;
+            B w[WN];
+    #pragma unroll
+            for (int k = 0; k < WN; ++k) w[k] = F(i - WO + k);
+            // row r of the system; `ends`: r may be a bounded system's
+            // first or last row (identity rows)
+            auto gen = [&](int r, bool ends, B &a, B &b, B &c, B &d) {
+                if (ends && bounded && (r == 0 || r == N - 1)) {
+                    a = B(0);
+                    b = B(1);
+                    c = B(0);
+                    d = r == 0 ? did0 : did1;
+                } else {
+                    // '+': cells i-2..i+2 = w[0..4]; '-': cells i+3..i-1 = w[5..1]
+                    // with the off-diagonals swapped (crweno5.cpp:335-338)
+                    constexpr bool m = S != 0;
+                    B lo, hi;
+                    if (SCH == SCHEME_H77)
+                        // '+': cells i-3..i+3 = w[0..6]; '-': cells i+4..i-2 = w[7..1]
+                        // (hccs77.cpp:282-291 swaps the couplings alike)
+                        h77_row(w[m ? 7 : 0], w[m ? 6 : 1], w[m ? 5 : 2], w[m ? 4 : 3],
+                                w[m ? 3 : 4], w[m ? 2 : 5], w[m ? 1 : 6], lo, b, hi, d);
+                    else if (SCH == SCHEME_HC)
+                        hc_row(m ? w[5] : w[0], m ? w[4] : w[1], m ? w[3] : w[2],
+                               m ? w[2] : w[3], m ? w[1] : w[4], lo, b, hi, d);
+                    else
+                        cr_row(m ? w[5] : w[0], m ? w[4] : w[1], m ? w[3] : w[2],
+                               m ? w[2] : w[3], m ? w[1] : w[4], lo, b, hi, d);
+                    a = m ? hi : lo;
+                    c = m ? lo : hi;
+                }
+            };
+            auto advance = [&]() {
+    #pragma unroll
+                for (int k = 0; k < WN - 1; ++k) w[k] = w[k + 1];
+                ++i;
+                w[WN - 1] = F(i + WN - 1 - WO);
+            };
+            B a0, b0, c0, d0;
+            gen(r0, true, a0, b0, c0, d0);
+            // forward: row j -> A x_first + x_j + C x_{j+1} = D.  Starting
+            // from (A, C, D) = (-1, 0, 0) makes row 1's update exact
+            // (b - a 0 = b, -a (-1) = a, d - a 0 = d), so every row takes
+            // the same code; only the last row can be an identity row.
+            B Ap = B(-1), Cp = B(0), Dp = B(0);
+            auto eliminate = [&](int j, B a, B b, B c, B d) {
+                const B bpv = b - a * Cp;
+                const B An = -a * Ap;
+                const B Dn = d - a * Dp;
+                const B r = rcp_(bpv);
+                Ap = An * r;
+                Cp = c * r;
+                Dp = Dn * r;
+                wA[j * 32 + lane] = Ap;
+                wC[j * 32 + lane] = Cp;
+                wD[j * 32 + lane] = Dp;
+            };
+            for (int j = 1; j < L - 1; ++j) {
+                advance();
+                B a, b, c, d;
+                gen(r0 + j, false, a, b, c, d);
+                eliminate(j, a, b, c, d);
+            }
+            {
+                advance();
+                B a, b, c, d;
+                gen(r0 + L - 1, true, a, b, c, d);
+                eliminate(L - 1, a, b, c, d);
+            }
+            la = Ap;
+            lc = Cp;
+            ld = Dp;
+            // backward: row j -> A x_first + x_j + C x_last = D
+            B bf = b0, cf = c0, df = d0;
+            if (L >= 3) {
+                B An = wA[(L - 2) * 32 + lane], Cn = wC[(L - 2) * 32 + lane];
+                B Dn = wD[(L - 2) * 32 + lane];
+                for (int j = L - 3; j >= 1; --j) {
+                    const B k = wC[j * 32 + lane];
+                    An = wA[j * 32 + lane] - k * An;
+                    Cn = -k * Cn;
+                    Dn = wD[j * 32 + lane] - k * Dn;
+                    wA[j * 32 + lane] = An;
+                    wC[j * 32 + lane] = Cn;
+                    wD[j * 32 + lane] = Dn;
+                }
+                // row 0 minus c0 x (row 1)
+                bf = b0 - c0 * An;
+                cf = -c0 * Cn;
+                df = d0 - c0 * Dn;
+            }
+            const B r = rcp_(bf);
+            fa = a0 * r;
+            fc = cf * r;
+            fd = df * r;
+        }
+    };
+    if (sg == 0)
+        segment(std::integral_constant<int, 0>{});
+    else
+        segment(std::integral_constant<int, 1>{});
+    // The 2P segment-end unknowns couple as
+    //   fa x_last(l-1) + x_first(l) + fc x_last(l)  = fd   (lane l's first)
+    //   la x_first(l)  + x_last(l)  + lc x_first(l+1) = ld (lane l's last)
+    // (neighbour lanes wrap for periodic lines; for bounded lines lane
+    // 0's fa and lane P-1's lc are 0: identity end rows).  Substituting
+    // the first rows into the last rows leaves a tridiagonal system in
+    // the P unknowns x_last alone,
+    //   -la fa x_last(l-1) + (1 - la fc - lc fa') x_last(l) - lc fc' x_last(l+1)
+    //     = ld - la fd - lc fd'          (' : lane l+1),
+    // solved by parallel cyclic reduction with shuffles (log2 P levels
+    // of one row each, instead of log2 2P levels of two rows); then
+    // x_first(l) = fd - fa x_last(l-1) - fc x_last(l).
+    B xf, xl;
+    {
+        // P is a power of two: lane indices wrap with a mask
+        const int pm = P - 1;
+        const int lp1 = (hl + 1) & pm, lm1 = (hl - 1) & pm;
+        const B nfa = shfl(fa, lp1), nfc = shfl(fc, lp1), nfd = shfl(fd, lp1);
+        const B r = rcp_(B(1) - la * fc - lc * nfa);
+        B ra = -la * fa * r, rc = -lc * nfc * r, rd = (ld - la * fd - lc * nfd) * r;
+#pragma unroll
+        for (int s = 1; s < kCrLanes; s <<= 1) {
+            if (s >= P) break;  // warp-uniform
+            const int sm = (hl - s) & pm, sp = (hl + s) & pm;
+            B ma = shfl(ra, sm), mc = shfl(rc, sm), md = shfl(rd, sm);
+            B pa = shfl(ra, sp), pc = shfl(rc, sp), pd = shfl(rd, sp);
+            if (bounded && hl < s) ma = mc = md = B(0);
+            if (bounded && hl + s >= P) pa = pc = pd = B(0);
+            pcr_update(ra, rc, rd, ma, mc, md, pa, pc, pd);
+        }
+        // after the last level each row couples only to itself
+        // (periodic) or to nothing (bounded)
+        xl = rd * rcp_(B(1) + ra + rc);
+        const B xlm = shfl(xl, lm1);
+        xf = fd - fa * xlm - fc * xl;
+    }
+    __syncwarp();  // every lane has read its staged fluxes
+    if (act) {
+        const int off = bounded ? H : 0;
+        myF[r0 + off] = xf;
+        myF[r1 + off] = xl;
+        for (int j = 1; j < L - 1; ++j)
+            myF[r0 + j + off] =
+                wD[j * 32 + lane] - wA[j * 32 + lane] * xf - wC[j * 32 + lane] * xl;
+        if (!bounded && hl == 0) myF[n] = xf;  // face n is face 0
+    }
+    if (xm >= 0) myF[xm] = xv;
+}
+
 // Work item (box, a, b, -): DIR 0: lines j = a*TL.., k = b; DIR 1: lines
 // i = a*TL.., k = b; DIR 2: lines i = a*TL.., j = b.
 // prim_mode (x lines only, whose blocks own whole lines): 0 reads the
@@ -215,11 +434,9 @@ __global__ void __launch_bounds__(kCrThreads, sizeof(B) == 8 ? 3 : 4)
     while (P < kCrLanes && 2 * P <= N / 2) P *= 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // warp w solves line w/2 of the tile for sign w%2 (0: +, 1: -)
-    const int line = warp >> 1, sg = warp & 1, hl = lane;
+    const int line = warp >> 1, sg = warp & 1;
     B *const myF = sF + (sg * kCrTL + line) * ls;  // cell c at [c + H]; later face m at [m]
     B *const wA = sRow + (size_t)warp * 3 * ms * 32;  // [j][lane]
-    B *const wC = wA + ms * 32;
-    B *const wD = wC + ms * 32;
     const B inv_d = B(bp.inv_d[DIR]);
 
     if (DIR == 0 && prim_mode != 0) {  // block-uniform
@@ -310,212 +527,7 @@ __global__ void __launch_bounds__(kCrThreads, sizeof(B) == 8 ? 3 : 4)
         __syncthreads();
 
         if (l0 + line < nl) {  // warp-uniform
-            // explicit faces of the bounded system: 0..H-1 and n-H+1..n
-            int xm = -1;
-            B xv = B(0);
-            // segment of this lane: rows r0 .. r1 (at least 2)
-            const bool act = hl < P;
-            const int r0 = act ? (hl * N) / P : 0;
-            const int r1 = act ? ((hl + 1) * N) / P - 1 : 1;
-            const int L = r1 - r0 + 1;
-            B fa = B(0), fc = B(0), fd = B(0);  // reduced unit-diagonal row of x_first
-            B la = B(0), lc = B(0), ld = B(0);  // reduced unit-diagonal row of x_last
-            // the row work of one sign; the sign (warp-uniform) is a compile-time
-            // constant inside, so each warp runs code without sign selects
-            auto segment = [&](auto sign) {
-                constexpr int S = decltype(sign)::value;
-                auto F = [&](int c) -> B { return myF[c + H]; };
-                // the sign (warp-uniform) only selects which cells feed a
-                // stencil ('+' reads upwind from the left, '-' from the right)
-                constexpr int dir = S == 0 ? 1 : -1;
-                // explicit face m: WENO5-JS (crweno5.cpp:425-837), hccs's WENO7
-                // (hccs.cpp:538-980) or hccs77's WENO7-Z (hccs77.cpp:330-818)
-                auto js = [&](int m) -> B {
-                    if (SCH == SCHEME_HC || SCH == SCHEME_H77) {
-                        const int c0 = S == 0 ? m - 4 : m + 3;
-                        if (SCH == SCHEME_HC)
-                            return weno7_face_hc(F(c0), F(c0 + dir), F(c0 + 2 * dir),
-                                                 F(c0 + 3 * dir), F(c0 + 4 * dir), F(c0 + 5 * dir),
-                                                 F(c0 + 6 * dir));
-                        return weno7_face(F(c0), F(c0 + dir), F(c0 + 2 * dir), F(c0 + 3 * dir),
-                                          F(c0 + 4 * dir), F(c0 + 5 * dir), F(c0 + 6 * dir));
-                    }
-                    const int c0 = S == 0 ? m - 3 : m + 2;
-                    return weno5js_face(F(c0), F(c0 + dir), F(c0 + 2 * dir), F(c0 + 3 * dir),
-                                        F(c0 + 4 * dir));
-                };
-                // lanes 0..2H-1: the explicit faces; lanes 2H and 2H+1: the
-                // identity rows' values (faces H and n-H), passed to the lanes
-                // that own those rows, so the warp evaluates explicit faces once
-                B did0 = B(0), did1 = B(0);
-                if (bounded) {
-                    B v = B(0);
-                    if (hl < 2 * H + 2) {
-                        const int m = hl < H ? hl
-                                             : (hl < 2 * H ? n - 2 * H + 1 + hl
-                                                           : (hl == 2 * H ? H : n - H));
-                        v = js(m);
-                        if (hl < 2 * H) {
-                            xm = m;
-                            xv = v;
-                        }
-                    }
-                    did0 = shfl(v, 2 * H);
-                    did1 = shfl(v, 2 * H + 1);
-                }
-                if (act) {
-                    // window w[k] = F(i - WO + k) of the current row's cell i (face
-                    // i + 1): cells i-2..i+3 for the 5-cell rows, i-3..i+4 for
-                    // hccs77's 7-cell rows
-                    constexpr int WN = SCH == SCHEME_H77 ? 8 : 6, WO = SCH == SCHEME_H77 ? 3 : 2;
-                    int i = bounded ? r0 + H - 1 : r0 - 1;
-                    B w[WN];
-    #pragma unroll
-                    for (int k = 0; k < WN; ++k) w[k] = F(i - WO + k);
-                    // row r of the system; `ends`: r may be a bounded system's
-                    // first or last row (identity rows)
-                    auto gen = [&](int r, bool ends, B &a, B &b, B &c, B &d) {
-                        if (ends && bounded && (r == 0 || r == N - 1)) {
-                            a = B(0);
-                            b = B(1);
-                            c = B(0);
-                            d = r == 0 ? did0 : did1;
-                        } else {
-                            // '+': cells i-2..i+2 = w[0..4]; '-': cells i+3..i-1 = w[5..1]
-                            // with the off-diagonals swapped (crweno5.cpp:335-338)
-                            constexpr bool m = S != 0;
-                            B lo, hi;
-                            if (SCH == SCHEME_H77)
-                                // '+': cells i-3..i+3 = w[0..6]; '-': cells i+4..i-2 = w[7..1]
-                                // (hccs77.cpp:282-291 swaps the couplings alike)
-                                h77_row(w[m ? 7 : 0], w[m ? 6 : 1], w[m ? 5 : 2], w[m ? 4 : 3],
-                                        w[m ? 3 : 4], w[m ? 2 : 5], w[m ? 1 : 6], lo, b, hi, d);
-                            else if (SCH == SCHEME_HC)
-                                hc_row(m ? w[5] : w[0], m ? w[4] : w[1], m ? w[3] : w[2],
-                                       m ? w[2] : w[3], m ? w[1] : w[4], lo, b, hi, d);
-                            else
-                                cr_row(m ? w[5] : w[0], m ? w[4] : w[1], m ? w[3] : w[2],
-                                       m ? w[2] : w[3], m ? w[1] : w[4], lo, b, hi, d);
-                            a = m ? hi : lo;
-                            c = m ? lo : hi;
-                        }
-                    };
-                    auto advance = [&]() {
-    #pragma unroll
-                        for (int k = 0; k < WN - 1; ++k) w[k] = w[k + 1];
-                        ++i;
-                        w[WN - 1] = F(i + WN - 1 - WO);
-                    };
-                    B a0, b0, c0, d0;
-                    gen(r0, true, a0, b0, c0, d0);
-                    // forward: row j -> A x_first + x_j + C x_{j+1} = D.  Starting
-                    // from (A, C, D) = (-1, 0, 0) makes row 1's update exact
-                    // (b - a 0 = b, -a (-1) = a, d - a 0 = d), so every row takes
-                    // the same code; only the last row can be an identity row.
-                    B Ap = B(-1), Cp = B(0), Dp = B(0);
-                    auto eliminate = [&](int j, B a, B b, B c, B d) {
-                        const B bpv = b - a * Cp;
-                        const B An = -a * Ap;
-                        const B Dn = d - a * Dp;
-                        const B r = rcp_(bpv);
-                        Ap = An * r;
-                        Cp = c * r;
-                        Dp = Dn * r;
-                        wA[j * 32 + lane] = Ap;
-                        wC[j * 32 + lane] = Cp;
-                        wD[j * 32 + lane] = Dp;
-                    };
-                    for (int j = 1; j < L - 1; ++j) {
-                        advance();
-                        B a, b, c, d;
-                        gen(r0 + j, false, a, b, c, d);
-                        eliminate(j, a, b, c, d);
-                    }
-                    {
-                        advance();
-                        B a, b, c, d;
-                        gen(r0 + L - 1, true, a, b, c, d);
-                        eliminate(L - 1, a, b, c, d);
-                    }
-                    la = Ap;
-                    lc = Cp;
-                    ld = Dp;
-                    // backward: row j -> A x_first + x_j + C x_last = D
-                    B bf = b0, cf = c0, df = d0;
-                    if (L >= 3) {
-                        B An = wA[(L - 2) * 32 + lane], Cn = wC[(L - 2) * 32 + lane];
-                        B Dn = wD[(L - 2) * 32 + lane];
-                        for (int j = L - 3; j >= 1; --j) {
-                            const B k = wC[j * 32 + lane];
-                            An = wA[j * 32 + lane] - k * An;
-                            Cn = -k * Cn;
-                            Dn = wD[j * 32 + lane] - k * Dn;
-                            wA[j * 32 + lane] = An;
-                            wC[j * 32 + lane] = Cn;
-                            wD[j * 32 + lane] = Dn;
-                        }
-                        // row 0 minus c0 x (row 1)
-                        bf = b0 - c0 * An;
-                        cf = -c0 * Cn;
-                        df = d0 - c0 * Dn;
-                    }
-                    const B r = rcp_(bf);
-                    fa = a0 * r;
-                    fc = cf * r;
-                    fd = df * r;
-                }
-            };
-            if (sg == 0)
-                segment(std::integral_constant<int, 0>{});
-            else
-                segment(std::integral_constant<int, 1>{});
-            // The 2P segment-end unknowns couple as
-            //   fa x_last(l-1) + x_first(l) + fc x_last(l)  = fd   (lane l's first)
-            //   la x_first(l)  + x_last(l)  + lc x_first(l+1) = ld (lane l's last)
-            // (neighbour lanes wrap for periodic lines; for bounded lines lane
-            // 0's fa and lane P-1's lc are 0: identity end rows).  Substituting
-            // the first rows into the last rows leaves a tridiagonal system in
-            // the P unknowns x_last alone,
-            //   -la fa x_last(l-1) + (1 - la fc - lc fa') x_last(l) - lc fc' x_last(l+1)
-            //     = ld - la fd - lc fd'          (' : lane l+1),
-            // solved by parallel cyclic reduction with shuffles (log2 P levels
-            // of one row each, instead of log2 2P levels of two rows); then
-            // x_first(l) = fd - fa x_last(l-1) - fc x_last(l).
-            B xf, xl;
-            {
-                // P is a power of two: lane indices wrap with a mask
-                const int pm = P - 1;
-                const int lp1 = (hl + 1) & pm, lm1 = (hl - 1) & pm;
-                const B nfa = shfl(fa, lp1), nfc = shfl(fc, lp1), nfd = shfl(fd, lp1);
-                const B r = rcp_(B(1) - la * fc - lc * nfa);
-                B ra = -la * fa * r, rc = -lc * nfc * r, rd = (ld - la * fd - lc * nfd) * r;
-#pragma unroll
-                for (int s = 1; s < kCrLanes; s <<= 1) {
-                    if (s >= P) break;  // warp-uniform
-                    const int sm = (hl - s) & pm, sp = (hl + s) & pm;
-                    B ma = shfl(ra, sm), mc = shfl(rc, sm), md = shfl(rd, sm);
-                    B pa = shfl(ra, sp), pc = shfl(rc, sp), pd = shfl(rd, sp);
-                    if (bounded && hl < s) ma = mc = md = B(0);
-                    if (bounded && hl + s >= P) pa = pc = pd = B(0);
-                    pcr_update(ra, rc, rd, ma, mc, md, pa, pc, pd);
-                }
-                // after the last level each row couples only to itself
-                // (periodic) or to nothing (bounded)
-                xl = rd * rcp_(B(1) + ra + rc);
-                const B xlm = shfl(xl, lm1);
-                xf = fd - fa * xlm - fc * xl;
-            }
-            __syncwarp();  // every lane has read its staged fluxes
-            if (act) {
-                const int off = bounded ? H : 0;
-                myF[r0 + off] = xf;
-                myF[r1 + off] = xl;
-                for (int j = 1; j < L - 1; ++j)
-                    myF[r0 + j + off] =
-                        wD[j * 32 + lane] - wA[j * 32 + lane] * xf - wC[j * 32 + lane] * xl;
-                if (!bounded && hl == 0) myF[n] = xf;  // face n is face 0
-            }
-            if (xm >= 0) myF[xm] = xv;
+            line_solve<B, SCH>(myF, wA, ms, n, N, P, bounded, sg, lane);
         }
         __syncthreads();
         // dF/dx of the tile's cells from F^ = F^+ + F^- (euler3d.cpp:23-56, 143-253)
@@ -611,6 +623,52 @@ cudaError_t launch_crweno(int sch, int dir, const BoxDev *boxes, const WorkItem 
     else
         launch_t<B, SCHEME_CR>(dir, boxes, items, nitems, in_slot, accumulate, nmax, ms, prim_mode,
                                smem, st);
+    return cudaGetLastError();
+}
+
+// nuc3d_reconstruct of the line-solve schemes: one warp per line, staged with
+// its halos in shared memory (coalesced both ways) and solved as the sweeps
+// solve theirs.  Bound by instruction issue like them.  192 x 128 x 96 cells,
+// one direction: crweno5 253 -> 29 us, hccs 174 -> 33, hccs77 255 -> 54 against
+// a thread per line (k_op_crweno, k_op_hccs), whose serial recurrences leave
+// 12288 threads waiting on strided loads.
+template <int SCH>
+__global__ void __launch_bounds__(256)
+    k_op_lines(int sg, int nx, long long lines, int ms, int N, int P, const double *__restrict__ in,
+               const double *__restrict__ hl, const double *__restrict__ hr,
+               double *__restrict__ out) {
+    constexpr int H = scheme_halo(SCH);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long line = (long long)blockIdx.x * (blockDim.x >> 5) + warp;
+    if (line >= lines) return;
+    const int nst = nx + 2 * H;
+    double *const f = reinterpret_cast<double *>(smem_raw) + (size_t)warp * (nst + 3 * ms * 32);
+    for (int c = lane; c < nst; c += 32) {
+        const int i = c - H;
+        f[c] = i < 0 ? hl[H * line + c] : (i >= nx ? hr[H * line + i - nx] : in[nx * line + i]);
+    }
+    __syncwarp();
+    line_solve<double, SCH>(f, f + nst, ms, nx, N, P, true, sg, lane);
+    __syncwarp();
+    for (int m = lane; m <= nx; m += 32) out[(nx + 1) * line + m] = f[m];
+}
+
+cudaError_t op_lines(int sch, int upwind, int nx, long long lines, const double *in,
+                     const double *hl, const double *hr, double *out, cudaStream_t st) {
+    const int ms = crweno_segment_rows(sch, nx, true), P = crweno_lanes(sch, nx, true);
+    const int N = line_unknowns(sch, nx, true);
+    const size_t per = sizeof(double) * (size_t)(nx + 2 * scheme_halo(sch) + 3 * ms * 32);
+    const size_t fit = (size_t)200 * 1024 / per;  // nx = 4096: 131 KB, one warp
+    const int warps = (int)(fit < 8 ? fit : 8);
+    const auto k = sch == SCHEME_HC    ? k_op_lines<SCHEME_HC>
+                   : sch == SCHEME_H77 ? k_op_lines<SCHEME_H77>
+                                       : k_op_lines<SCHEME_CR>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(per * warps));
+    if (e != cudaSuccess) return e;
+    k<<<(unsigned)((lines + warps - 1) / warps), 32 * warps, per * warps, st>>>(
+        upwind > 0 ? 0 : 1, nx, lines, ms, N, P, in, hl, hr, out);
     return cudaGetLastError();
 }
 

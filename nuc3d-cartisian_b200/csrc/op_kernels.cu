@@ -306,6 +306,13 @@ cudaError_t op_reconstruct(int scheme, int upwind, unsigned quirks, int nx, long
                            const double *in, const double *hl, const double *hr, double *out,
                            cudaStream_t st) {
     if (scheme == SCHEME_CR || scheme == SCHEME_HC || scheme == SCHEME_H77) {
+        // A warp per line (crweno_kernels.cu) unless the lines are short, so that
+        // few of its lanes have rows, and many enough to fill the GPU with a
+        // thread each.  crweno5, a thread / a warp per line, us: 16 cells x 65536
+        // lines 48 / 64, 32 x 32768 55 / 46, 48 x 16384 69 / 22, 192 x 12288
+        // 253 / 29, 16 x 64 28 / 10 (hccs 32 x 32768 51 / 54, hccs77 59 / 89).
+        if (nx >= 48 || lines <= 16384)
+            return op_lines(scheme, upwind, nx, lines, in, hl, hr, out, st);
         double *scratch = nullptr;
         size_t bytes = sizeof(double) * 2 * (size_t)nx * (size_t)lines;
         cudaError_t e = cudaMallocAsync(&scratch, bytes, st);

@@ -14,6 +14,9 @@ struct RK5 {
 cudaError_t op_reconstruct(int scheme, int upwind, unsigned quirks, int nx, long long lines,
                            const double *in, const double *hl, const double *hr, double *out,
                            cudaStream_t st);
+// the line-solve schemes' reconstruction, one warp per line (crweno_kernels.cu)
+cudaError_t op_lines(int sch, int upwind, int nx, long long lines, const double *in,
+                     const double *hl, const double *hr, double *out, cudaStream_t st);
 // CRWENO5 line solve with caller-provided scratch (2 * nx * lines doubles).
 cudaError_t op_crweno_into(int upwind, int nx, long long lines, const double *in,
                            const double *hl, const double *hr, double *out, double *scratch,
