@@ -561,7 +561,7 @@ int Engine::rebuild() {
         for (int d = 0; d < 3; ++d) per_stage += r_cr_[c][d].n > 0;
     launches_per_step_ = 3 * per_stage + 3;  // + clear_eig, dt, residual
     for (const EngineBox &b : boxes_)
-        if (b.live && b.dev.active && b.force_mem) launches_per_step_ += 3 * 8;  // forcing passes
+        if (b.live && b.dev.active && b.force_mem) launches_per_step_ += 3 * 6;  // forcing passes
     dirty_ = false;
     return NUC3D_OK;
 }

@@ -23,7 +23,6 @@ struct ForceParams {
 struct ForceScratch {
     double2 *tx, *ty, *tz;  // twiddles exp(+i 2 pi k j / n), k = -K..K
     double2 *a, *b, *fh;    // transform passes and the forcing spectrum
-    double *partials;       // per-line sums of f.u
     double *scal;           // E_s, E_c, theta (band: the gain P / (2 E_b)), <f.u>
 };
 
