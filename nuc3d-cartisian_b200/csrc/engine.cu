@@ -441,7 +441,7 @@ int Engine::rebuild() {
     const bool mixed = precision_ == NUC3D_MIXED;
     std::vector<BoxDev> table(boxes_.size());
     std::vector<WorkItem> prim, st25[kVisClasses], inv[kSchemes][3][kInvTileClasses],
-        march[kSchemes][3], cr[kLineSchemes][3];
+        march[kSchemes][3], thomas[3], cr[kLineSchemes][3];
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d) march_nmax_[s][d] = 0;
     const int crtl = crweno_tile_lines();
@@ -474,6 +474,11 @@ int Engine::rebuild() {
             if (line_slot(s) >= 0) {
                 const int c = line_slot(s);
                 const bool bounded = s != SCHEME_CR || (p.quirks & QK_CRWENO_BOUNDED) != 0;
+                if (thomas_lines_of(s, d, mixed, bounded)) {
+                    const long long lines = p.N / p.n[d];
+                    for (int g = 0; g * 32LL < lines; ++g) thomas[d].push_back({id, g, 0, 0});
+                    continue;
+                }
                 cr_nmax_[c][d] = std::max(cr_nmax_[c][d], p.n[d]);
                 cr_ms_[c][d] = std::max(cr_ms_[c][d], crweno_segment_rows(s, p.n[d], bounded));
                 auto &L = cr[c][d];
@@ -527,6 +532,7 @@ int Engine::rebuild() {
             for (int tc = 0; tc < kInvTileClasses; ++tc) append(inv[s][d][tc], r_inv_[s][d][tc]);
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d) append(march[s][d], r_march_[s][d]);
+    for (int d = 0; d < 3; ++d) append(thomas[d], r_thomas_[d]);
     for (int c = 0; c < kLineSchemes; ++c)
         for (int d = 0; d < 3; ++d) append(cr[c][d], r_cr_[c][d]);
     if ((int)boxes_.size() > d_boxes_cap_) {
@@ -559,6 +565,7 @@ int Engine::rebuild() {
         for (int d = 0; d < 3; ++d) per_stage += has_sweep(s, d);
     for (int c = 0; c < kLineSchemes; ++c)
         for (int d = 0; d < 3; ++d) per_stage += r_cr_[c][d].n > 0;
+    for (int d = 0; d < 3; ++d) per_stage += r_thomas_[d].n > 0;
     launches_per_step_ = 3 * per_stage + 3;  // + clear_eig, dt, residual
     for (const EngineBox &b : boxes_)
         if (b.live && b.dev.active && b.force_mem) launches_per_step_ += 3 * 6;  // forcing passes
@@ -623,10 +630,7 @@ int Engine::enqueue_step_t(cudaStream_t st) {
             const int prim_mode = d == 0 ? (stage == 0 ? 2 : 1) : 0;
             for (int s = 0; s < kSchemes; ++s)
                 ECK((launch_sweep<B>(s, d, inv_variant[s][d], in, prim_mode, st)));
-            for (int c = 0; c < kLineSchemes; ++c)
-                ECK((launch_crweno<B>(kLineScheme[c], d, d_boxes_,
-                                      it + r_cr_[c][d].off, r_cr_[c][d].n, in, d > 0,
-                                      cr_nmax_[c][d], cr_ms_[c][d], prim_mode, st)));
+            ECK(launch_lines<B>(d, in, prim_mode, st));
             return NUC3D_OK;
         };
         if (int rc = sweeps(0)) return rc;
@@ -639,8 +643,11 @@ int Engine::enqueue_step_t(cudaStream_t st) {
         // forked stream, beside the y and z sweeps (an HBM- and
         // latency-bound kernel next to FP64-bound ones), and join before the
         // update.  Eager (profiled) steps keep one stream.
-        const bool fork = any_visc_ && fork_stream_ && st == cap_stream_;
-        if (any_visc_) {
+        // (Boxes whose line solves use the viscous fluxes as scratch: after the
+        // sweeps.)
+        const bool late = any_thomas();
+        const bool fork = any_visc_ && fork_stream_ && st == cap_stream_ && !late;
+        auto visc = [&]() -> int {
             ProfScope ps(this, NUC3D_PROF_VISC);
             cudaStream_t vs = st;
             if (fork) {
@@ -650,9 +657,14 @@ int Engine::enqueue_step_t(cudaStream_t st) {
             }
             ECK(launch_visc_classes<B>(pv(), vs));
             if (fork) ECK(cudaEventRecord(fork_ev_[1], fork_stream_));
-        }
+            return NUC3D_OK;
+        };
+        if (any_visc_ && !late)
+            if (int rc = visc()) return rc;
         for (int d = 1; d < 3; ++d)
             if (int rc = sweeps(d)) return rc;
+        if (any_visc_ && late)
+            if (int rc = visc()) return rc;
         ECK(enqueue_forcing<B>(st));
         if (fork) ECK(cudaStreamWaitEvent(st, fork_ev_[1], 0));
         {
@@ -666,6 +678,19 @@ int Engine::enqueue_step_t(cudaStream_t st) {
         ECK(launch_residual(d_boxes_, nb, st));
     }
     return NUC3D_OK;
+}
+
+template <typename B>
+cudaError_t Engine::launch_lines(int d, int in, int prim_mode, cudaStream_t st) {
+    for (int c = 0; c < kLineSchemes; ++c) {
+        const Range &r = r_cr_[c][d];
+        cudaError_t e = launch_crweno<B>(kLineScheme[c], d, d_boxes_, d_items_ + r.off, r.n, in,
+                                         d > 0, cr_nmax_[c][d], cr_ms_[c][d], prim_mode, st);
+        if (e != cudaSuccess) return e;
+    }
+    // (u_n is slot 0; the stages read slots 0, 1, 2 in turn)
+    return launch_thomas(d, d_boxes_, d_items_ + r_thomas_[d].off, r_thomas_[d].n, in,
+                         in == 2 ? 1 : 2, st);
 }
 
 template <typename B>
@@ -940,15 +965,12 @@ int Engine::enqueue_rhs_t(int id, double *const d_rhs[5]) {
     ECK(launch_clear_eig(d_boxes_, nb, stream_));
     ECK(launch_prim(d_boxes_, it + r_prim_.off, r_prim_.n, 0, 1, stream_));
     ECK(launch_dt(d_boxes_, nb, stream_));
-    if (any_visc_) ECK(launch_visc_classes<B>(pv(), stream_));
     for (int d = 0; d < 3; ++d) {
         for (int s = 0; s < kSchemes; ++s)
             ECK((launch_sweep<B>(s, d, inv_variant[s][d], 0, 0, stream_)));
-        for (int c = 0; c < kLineSchemes; ++c)
-            ECK((launch_crweno<B>(kLineScheme[c], d, d_boxes_, it + r_cr_[c][d].off,
-                                  r_cr_[c][d].n, 0, d > 0, cr_nmax_[c][d], cr_ms_[c][d], 0,
-                                  stream_)));
+        ECK(launch_lines<B>(d, 0, 0, stream_));
     }
+    if (any_visc_) ECK(launch_visc_classes<B>(pv(), stream_));
     ECK(enqueue_forcing<B>(stream_));
     StageArgs sa{-1, 0, 0, d_rhs_ptrs_};
     ECK(launch_update_classes<B>(pv(), sa, stream_));

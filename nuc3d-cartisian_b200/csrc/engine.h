@@ -141,6 +141,12 @@ private:
     Range r_march_[kSchemes][3];
     int march_nmax_[kSchemes][3] = {};
     bool has_sweep(int s, int d) const { return r_inv_[s][d][0].n > 0 || r_march_[s][d].n > 0; }
+    // line groups of the CRWENO5 sweeps that march (thomas_lines_of)
+    Range r_thomas_[3];
+    bool any_thomas() const { return r_thomas_[1].n > 0 || r_thomas_[2].n > 0; }
+    // the line-solve schemes' sweeps along d
+    template <typename B>
+    cudaError_t launch_lines(int d, int in, int prim_mode, cudaStream_t st);
     // variant v of the directional sweep of scheme s on this batch's boxes
     template <typename B>
     cudaError_t launch_sweep(int s, int d, int v, int in, int prim_mode, cudaStream_t st);

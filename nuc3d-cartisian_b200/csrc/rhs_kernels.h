@@ -156,6 +156,15 @@ constexpr bool marched(int scheme, int dir, bool mixed) {
 cudaError_t prepare_march_kernels();
 cudaError_t launch_march(int scheme, int dir, const BoxDev *boxes, const WorkItem *items,
                          int nitems, int nmax, int in_slot, int len, cudaStream_t st);
+// Bounded FP64 CRWENO5 sweeps along y and z by one thread per line and equation
+// (thomas_kernels.cu): work items as launch_march's.  free_slot: the state slot
+// that is neither u_n nor in_slot; the boxes' viscous fluxes and that slot are
+// scratch, so the viscous fluxes are computed after these sweeps.
+constexpr bool thomas_lines_of(int scheme, int dir, bool mixed, bool bounded) {
+    return !mixed && dir > 0 && scheme == SCHEME_CR && bounded;
+}
+cudaError_t launch_thomas(int dir, const BoxDev *boxes, const WorkItem *items, int nitems,
+                          int in_slot, int free_slot, cudaStream_t st);
 // raises the dynamic shared-memory limits of the 2.5-D stencil kernels
 cudaError_t prepare_stencil_kernels(bool mixed);
 // Stencil classes of the 2.5-D kernels: boxes whose three directions use cd6
