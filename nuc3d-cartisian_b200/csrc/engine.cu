@@ -237,6 +237,27 @@ __global__ void k_export_flags(FlagPtrs f, unsigned *out) {
 
 Engine::Engine(int precision, cudaStream_t stream) : precision_(precision), stream_(stream) {
     cudaGetDevice(&device_);
+    std::fill(pencil_of_class, pencil_of_class + kPencilClasses, (signed char)-1);
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device_;
+    if (cudaMemPoolCreate(&pool_, &props) != cudaSuccess) {
+        pool_ = nullptr;
+        cudaGetLastError();
+    }
+    set_pool_keep();
+}
+
+void Engine::set_pool_keep() {
+    if (!pool_) return;
+    unsigned long long keep = box_bytes_ + kPoolKeep;
+    cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+
+cudaError_t Engine::device_alloc(void **p, size_t bytes) {
+    return pool_ ? cudaMallocFromPoolAsync(p, bytes, pool_, stream_)
+                 : cudaMallocAsync(p, bytes, stream_);
 }
 
 Engine::~Engine() {
@@ -258,6 +279,8 @@ Engine::~Engine() {
     if (d_rhs_ptrs_) cudaFreeAsync(d_rhs_ptrs_, stream_);
     if (d_stats_) cudaFreeAsync(d_stats_, stream_);
     cudaStreamSynchronize(stream_);
+    spectra_plan_.release();
+    if (pool_) cudaMemPoolDestroy(pool_);
     for (cudaEvent_t e : ev_pool_) cudaEventDestroy(e);
     for (cudaEvent_t e : copy_ev_)
         if (e) cudaEventDestroy(e);
@@ -287,9 +310,9 @@ int Engine::add_box(const nuc3d_box_desc &d, int *id) {
     const long long np = pad32(b.dev.p.N);
     const size_t bs = bulk_size(precision_);
     const size_t bytes = sizeof(double) * 21 * (size_t)np + bs * 14 * (size_t)np + kSmallBytes;
-    cudaError_t e = cudaMallocAsync(&b.mem, bytes, stream_);
+    cudaError_t e = device_alloc(&b.mem, bytes);
     if (e == cudaSuccess && d.forcing != NUC3D_FORCING_NONE)
-        e = cudaMallocAsync(&b.force_mem, forcing_scratch_bytes(b.dev.p, d.forcing_k), stream_);
+        e = device_alloc(&b.force_mem, forcing_scratch_bytes(b.dev.p, d.forcing_k));
     if (e != cudaSuccess) {
         if (b.mem) cudaFreeAsync(b.mem, stream_);
         cudaGetLastError();
@@ -307,6 +330,7 @@ int Engine::add_box(const nuc3d_box_desc &d, int *id) {
     b.dev.sc = reinterpret_cast<StepScalars *>(sm + 256);
     b.dev.active = 1;
     b.live = true;
+    b.bytes = bytes + (b.force_mem ? forcing_scratch_bytes(b.dev.p, d.forcing_k) : 0);
     ECK(cudaMemsetAsync(b.mem, 0, bytes, stream_));
     // sc->cfl = 0.5 (the stream-ordered memset above runs first)
     static const double half = 0.5;
@@ -338,6 +362,8 @@ int Engine::add_box(const nuc3d_box_desc &d, int *id) {
     }
     *id = slot;
     dirty_ = true;
+    box_bytes_ += b.bytes;
+    set_pool_keep();
     return NUC3D_OK;
 }
 
@@ -347,6 +373,8 @@ int Engine::remove_box(int id) {
     EngineBox &b = boxes_[id];
     ECK(cudaFreeAsync(b.mem, stream_));
     if (b.force_mem) ECK(cudaFreeAsync(b.force_mem, stream_));
+    box_bytes_ -= b.bytes;
+    set_pool_keep();
     b = EngineBox();
     dirty_ = true;
     return NUC3D_OK;
@@ -539,13 +567,13 @@ int Engine::rebuild() {
         if (d_boxes_) ECK(cudaFreeAsync(d_boxes_, stream_));
         if (d_rhs_ptrs_) ECK(cudaFreeAsync(d_rhs_ptrs_, stream_));
         d_boxes_cap_ = std::max<int>(8, (int)boxes_.size() * 2);
-        ECK(cudaMallocAsync(&d_boxes_, sizeof(BoxDev) * d_boxes_cap_, stream_));
-        ECK(cudaMallocAsync(&d_rhs_ptrs_, sizeof(double *) * 5 * d_boxes_cap_, stream_));
+        ECK(device_alloc(&d_boxes_, sizeof(BoxDev) * d_boxes_cap_));
+        ECK(device_alloc(&d_rhs_ptrs_, sizeof(double *) * 5 * d_boxes_cap_));
     }
     if (all.size() > d_items_cap_) {
         if (d_items_) ECK(cudaFreeAsync(d_items_, stream_));
         d_items_cap_ = std::max<size_t>(1024, all.size() * 5 / 4);
-        ECK(cudaMallocAsync(&d_items_, sizeof(WorkItem) * d_items_cap_, stream_));
+        ECK(device_alloc(&d_items_, sizeof(WorkItem) * d_items_cap_));
     }
     if (!table.empty())
         ECK(cudaMemcpyAsync(d_boxes_, table.data(), sizeof(BoxDev) * table.size(),
@@ -745,12 +773,11 @@ int Engine::enqueue_step(cudaStream_t s) {
     return precision_ == NUC3D_MIXED ? enqueue_step_t<float>(s) : enqueue_step_t<double>(s);
 }
 
-// Picks the run length of the directional sweep per scheme and direction,
-// and the pencil depth of the 2.5-D stencil kernels, by timing every variant
-// on this batch's own work lists: the sweeps on the first step after a
-// rebuild that brings a new (scheme, direction) pair, the depth on the first
-// step and whenever the active cells have moved past 2x (or 1/2x) of those
-// it was tuned at.  The sweeps only write the RHS accumulator (and the x
+// Picks the variant of the directional sweep per scheme and direction, and the
+// pencil depth of the 2.5-D stencil kernels, by timing every variant on this
+// batch's own work lists: the sweeps on the first step after a rebuild that
+// brings a new (scheme, direction) pair, the depth on the first step in each
+// power of four of active cells.  The sweeps only write the RHS accumulator (and the x
 // sweep the primitives, with the values they already hold) and the
 // viscous-flux kernel the viscous fluxes, which every stage recomputes; the
 // update is timed as a first stage, which writes only the u1 slot that the
@@ -768,10 +795,14 @@ int Engine::autotune() {
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d)
             need_sweep = need_sweep || (has_sweep(s, d) && inv_variant[s][d] < 0);
-    const bool need_pencil =
-        (r_25d_[0].n > 0 || r_25d_[1].n > 0) &&
-        (pencil_variant < 0 || 2 * active_cells_ < pencil_tuned_cells ||
-                            active_cells_ > 2 * pencil_tuned_cells);
+    const bool stencils = r_25d_[0].n > 0 || r_25d_[1].n > 0;
+    int cls = 0;  // size class: floor(log4(active cells))
+    while (cls + 1 < kPencilClasses && (active_cells_ >> (2 * (cls + 1))) > 0) ++cls;
+    const bool need_pencil = stencils && pencil_of_class[cls] < 0;
+    if (stencils && !need_pencil && pencil_variant != pencil_of_class[cls]) {
+        pencil_variant = pencil_of_class[cls];
+        invalidate_graph();
+    }
     if (!need_sweep && !need_pencil) return NUC3D_OK;
     // NUC3D_SWEEP_RUN=1|2|4 pins the run length (32-cell tiles; with
     // NUC3D_SWEEP_TILE=64, runs of 2 or 4 on 64-cell tiles) and
@@ -799,7 +830,7 @@ int Engine::autotune() {
             pencil_variant = 0;
             for (int v = 0; v < kPencils; ++v)
                 if (kPencilDepths[v] == want) pencil_variant = v;
-            pencil_tuned_cells = active_cells_;
+            pencil_of_class[cls] = (signed char)pencil_variant;
             tune_pencil = false;
         }
     }
@@ -853,10 +884,12 @@ int Engine::autotune() {
     if (tune_pencil && rc == NUC3D_OK) {
         int best = 0;
         for (int v = 0; v < kPencils && rc == NUC3D_OK; ++v) {
-            // a short depth only where depth 16 makes few blocks and the
-            // next longer depth was the best so far
+            // 64 planes only where 16 are slower than 32; a short depth only
+            // where depth 16 makes few blocks and the next longer depth was
+            // the best so far
             const int longer = v == 3 ? 1 : v - 1;
-            if (v > 2 && (pencil_blocks(1) > kPencilShortBlocks || best != longer)) {
+            if ((v == 2 && best == 1) ||
+                (v > 2 && (pencil_blocks(1) > kPencilShortBlocks || best != longer))) {
                 pencil_tune_ms[v] = 0.0;
                 continue;
             }
@@ -874,7 +907,7 @@ int Engine::autotune() {
             if (ms < pencil_tune_ms[best]) best = v;
         }
         pencil_variant = best;
-        pencil_tuned_cells = active_cells_;
+        pencil_of_class[cls] = (signed char)best;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -1028,7 +1061,7 @@ int Engine::init_state(int id, const nuc3d_init_desc &in, double info[3]) {
     void *scratch = nullptr;
     double *d_sums = nullptr;
     const size_t bytes = hit_scratch_bytes(p, in.k_peak);
-    cudaError_t e = cudaMallocAsync(&scratch, bytes + 256, stream_);
+    cudaError_t e = device_alloc(&scratch, bytes + 256);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return set_last_error(NUC3D_ERR_NOMEM, "device allocation of the HIT scratch failed");
@@ -1076,7 +1109,7 @@ int Engine::stats(int id, double out[26]) {
     }
     EngineBox &b = boxes_[id];
     if (!b.dev.active) return set_last_error(NUC3D_ERR_INVALID, "box is not active");
-    if (!d_stats_) ECK(cudaMallocAsync(&d_stats_, sizeof(double) * stats_scratch_doubles(), stream_));
+    if (!d_stats_) ECK(device_alloc(&d_stats_, sizeof(double) * stats_scratch_doubles()));
     // primitives of U[0] into W (scratch between steps), then the sums
     ECK(launch_prim(d_boxes_, d_items_ + r_prim_.off + b.prim_off, b.prim_n, 0, 0, stream_));
     ECK(launch_stats(b.dev, d_stats_, stream_));
@@ -1100,30 +1133,34 @@ int Engine::spectra(int id, double *out, int *kmax_out) {
     *kmax_out = kmax;
     if (!out) return NUC3D_OK;
     if (!b.dev.active) return set_last_error(NUC3D_ERR_INVALID, "box is not active");
+    // the plan is kept for the next call; its work area, the fields and the
+    // result are one allocation of this call
     void *scratch = nullptr;
-    double *d_out = nullptr;
-    if (cudaMallocAsync(&scratch, spectra_scratch_bytes(b.dev.p), stream_) != cudaSuccess) {
-        cudaGetLastError();
-        return set_last_error(NUC3D_ERR_NOMEM, "no device memory for the spectra scratch");
-    }
-    int rc = NUC3D_OK;
-    int fft_status = 0;
-    cudaError_t e = cudaMallocAsync(&d_out, sizeof(double) * kSpectra * kmax, stream_);
-    if (e == cudaSuccess)
+    int fft_status = spectra_plan_.prepare(b.dev.p, stream_);
+    if (fft_status == 0) {
+        cudaError_t e = device_alloc(&scratch, spectra_scratch_bytes(b.dev.p, spectra_plan_.work));
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return set_last_error(NUC3D_ERR_NOMEM, "no device memory for the spectra scratch");
+        }
         e = launch_prim(d_boxes_, d_items_ + r_prim_.off + b.prim_off, b.prim_n, 0, 0, stream_);
-    if (e == cudaSuccess) e = launch_spectra(b.dev, scratch, d_out, &fft_status, stream_);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(out, d_out, sizeof(double) * kSpectra * kmax, cudaMemcpyDeviceToHost,
-                            stream_);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
-    if (fft_status != 0)
-        rc = set_last_error(NUC3D_ERR_CUDA, ("cuFFT failed with status " +
-                                             std::to_string(fft_status)).c_str());
-    else if (e != cudaSuccess)
-        rc = set_last_error(NUC3D_ERR_CUDA, cudaGetErrorString(e));
-    cudaFreeAsync(scratch, stream_);
-    if (d_out) cudaFreeAsync(d_out, stream_);
-    return rc;
+        double *d_out = nullptr;
+        if (e == cudaSuccess)
+            e = launch_spectra(b.dev, spectra_plan_, scratch, &d_out, &fft_status, stream_);
+        if (e == cudaSuccess && fft_status == 0)
+            e = cudaMemcpyAsync(out, d_out, sizeof(double) * kSpectra * kmax,
+                                cudaMemcpyDeviceToHost, stream_);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
+        cudaFreeAsync(scratch, stream_);
+        if (e != cudaSuccess && fft_status == 0)
+            return set_last_error(NUC3D_ERR_CUDA, cudaGetErrorString(e));
+    }
+    if (fft_status != 0) {
+        spectra_plan_.release();
+        return set_last_error(NUC3D_ERR_CUDA, ("cuFFT failed with status " +
+                                               std::to_string(fft_status)).c_str());
+    }
+    return NUC3D_OK;
 }
 
 int Engine::sync_and_check(int id) {

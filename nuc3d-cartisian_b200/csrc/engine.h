@@ -11,6 +11,7 @@
 
 #include "nuc3d_b200.h"
 #include "rhs_kernels.h"
+#include "spectra_kernels.h"
 
 namespace nuc3d {
 
@@ -20,6 +21,7 @@ struct EngineBox {
     int prim_off = 0, prim_n = 0;  // the box's k_prim work items (set by rebuild)
     void *mem = nullptr;   // one stream-ordered allocation holding all fields
     void *force_mem = nullptr;  // spectral forcing scratch (forced boxes only)
+    size_t bytes = 0;      // of mem and force_mem
     double cfl = 0.5;
     long long steps = 0;   // host mirror of the device step counter
     bool live = false;     // slot in use
@@ -87,11 +89,13 @@ public:
     }
     // autotuned pencil depth of the 2.5-D stencil kernels: index into
     // kPencilDepths (-1: not tuned yet), the measured milliseconds of one
-    // viscous-flux + update pass per depth, and the active cells it was tuned
-    // at (a batch that grows or shrinks past 2x is tuned again)
+    // viscous-flux + update pass per depth of the last tuning, and the depth
+    // found for each power of four of active cells (a batch that grows or
+    // shrinks into a size class it has been in takes that class's depth)
     int pencil_variant = -1;
     double pencil_tune_ms[kPencils] = {};
-    long long pencil_tuned_cells = 0;
+    static constexpr int kPencilClasses = 20;
+    signed char pencil_of_class[kPencilClasses];
 
     static long long box_bytes(const nuc3d_box_desc &d);
     static int validate(const nuc3d_box_desc &d, std::string *why);
@@ -118,6 +122,21 @@ private:
     cudaError_t launch_update_classes(int v, StageArgs sa, cudaStream_t st);
     void invalidate_graph();
     int autotune();
+
+    // Device memory of this engine comes from its own stream-ordered pool, which
+    // keeps up to kPoolKeep bytes of what it frees (the next box or spectra call
+    // then maps no memory) and is destroyed with the engine.  The pool's release
+    // threshold counts what is in use too, so it follows the boxes' bytes.
+    static constexpr unsigned long long kPoolKeep = 256ull << 20;
+    unsigned long long box_bytes_ = 0;
+    void set_pool_keep();
+    cudaError_t device_alloc(void **p, size_t bytes);
+    template <typename T>
+    cudaError_t device_alloc(T **p, size_t bytes) {
+        return device_alloc(reinterpret_cast<void **>(p), bytes);
+    }
+    cudaMemPool_t pool_ = nullptr;
+    SpectraPlan spectra_plan_;  // of the last box size asked for
 
     int precision_;
     cudaStream_t stream_;

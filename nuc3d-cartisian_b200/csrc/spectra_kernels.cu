@@ -6,7 +6,7 @@
 //                  |w|^2/2 (solveQ's fields, postproc.cpp:812-853, vorticity
 //                  from the differential scheme's gradients), density and
 //                  pressure, rows padded to 2 (nx/2 + 1) reals;
-//   cuFFT          one batched forward 3-D D2Z transform of the seven fields in
+//   cuFFT          forward 3-D D2Z transforms of the seven fields in
 //                  place (FFTW_FORWARD sign; the 1/N of fft.cpp:277-278 is
 //                  applied when binning).  The fields are real, so the modes
 //                  with kx < 0 are the conjugates of their mirrors and carry
@@ -200,51 +200,76 @@ __global__ void k_spec_reduce(const double *partials, int nblocks, int n, double
     if (lane == 0) out[t] = s;
 }
 
+size_t align256(size_t n) { return (n + 255) / 256 * 256; }
 size_t fields_bytes(const BoxParams &p) {
-    return sizeof(double2) * kSpectraFields * (size_t)(p.n[0] / 2 + 1) * p.n[1] * p.n[2];
+    return align256(sizeof(double2) * kSpectraFields * (size_t)(p.n[0] / 2 + 1) * p.n[1] * p.n[2]);
+}
+size_t partials_bytes(const BoxParams &p) {
+    return align256(sizeof(double) * (size_t)kSpecBlocks * kSpectra * spectra_kmax(p));
+}
+size_t out_bytes(const BoxParams &p) {
+    return align256(sizeof(double) * (size_t)kSpectra * spectra_kmax(p));
 }
 
 }  // namespace
 
-size_t spectra_scratch_bytes(const BoxParams &p) {
-    const int kmax = spectra_kmax(p);
-    return fields_bytes(p) + sizeof(double) * (size_t)kSpecBlocks * kSpectra * kmax;
+int SpectraPlan::prepare(const BoxParams &p, cudaStream_t st) {
+    cufftResult r = CUFFT_SUCCESS;
+    if (!made || n[0] != p.n[0] || n[1] != p.n[1] || n[2] != p.n[2]) {
+        release();
+        cufftHandle h;
+        r = cufftCreate(&h);
+        if (r != CUFFT_SUCCESS) return (int)r;
+        made = true;
+        handle = (int)h;
+        for (int d = 0; d < 3; ++d) n[d] = p.n[d];
+        // forward 3-D transforms (x fastest: dims nz, ny, nx), the seven fields
+        // together where they are small and launches count, else one by one
+        // with a work area of one field
+        batch = p.N <= 64 * 64 * 64 ? kSpectraFields : 1;
+        const long long nh = p.n[0] / 2 + 1, rows = (long long)p.n[1] * p.n[2];
+        long long dims[3] = {p.n[2], p.n[1], p.n[0]}, real[3] = {p.n[2], p.n[1], 2 * nh},
+                  half[3] = {p.n[2], p.n[1], nh};
+        r = cufftSetAutoAllocation(h, 0);
+        if (r == CUFFT_SUCCESS)
+            r = cufftMakePlanMany64(h, 3, dims, real, 1, 2 * nh * rows, half, 1, nh * rows,
+                                    CUFFT_D2Z, batch, &work);
+    }
+    if (r == CUFFT_SUCCESS) r = cufftSetStream((cufftHandle)handle, st);
+    return (int)r;
 }
 
-cudaError_t launch_spectra(const BoxDev &b, void *scratch, double *d_out, int *fft_status,
-                           cudaStream_t st) {
+void SpectraPlan::release() {
+    if (made) cufftDestroy((cufftHandle)handle);
+    *this = SpectraPlan();
+}
+
+size_t spectra_scratch_bytes(const BoxParams &p, size_t work) {
+    return fields_bytes(p) + partials_bytes(p) + out_bytes(p) + work;
+}
+
+cudaError_t launch_spectra(const BoxDev &b, const SpectraPlan &plan, void *scratch,
+                           double **d_out, int *fft_status, cudaStream_t st) {
     const BoxParams &p = b.p;
     const int kmax = spectra_kmax(p);
-    double *F = static_cast<double *>(scratch);
-    double *partials = reinterpret_cast<double *>(static_cast<char *>(scratch) + fields_bytes(p));
-    *fft_status = CUFFT_SUCCESS;
+    char *c = static_cast<char *>(scratch);
+    double *F = reinterpret_cast<double *>(c);
+    double *partials = reinterpret_cast<double *>(c += fields_bytes(p));
+    double *out = reinterpret_cast<double *>(c += partials_bytes(p));
+    *d_out = out;
     if (diff_reach(p) == 3)
         k_spec_fields<3><<<4 * 148, kThreads, 0, st>>>(b, F);
     else
         k_spec_fields<4><<<4 * 148, kThreads, 0, st>>>(b, F);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    // forward 3-D transforms of the seven fields (x fastest: dims nz, ny, nx)
-    cufftHandle plan;
-    const long long nh = p.n[0] / 2 + 1, rows = (long long)p.n[1] * p.n[2];
-    long long dims[3] = {p.n[2], p.n[1], p.n[0]}, real[3] = {p.n[2], p.n[1], 2 * nh},
-              half[3] = {p.n[2], p.n[1], nh};
-    size_t work = 0;
-    cufftResult r = cufftCreate(&plan);
-    if (r == CUFFT_SUCCESS) {
-        r = cufftMakePlanMany64(plan, 3, dims, real, 1, 2 * nh * rows, half, 1, nh * rows,
-                                CUFFT_D2Z, kSpectraFields, &work);
-        if (r == CUFFT_SUCCESS) r = cufftSetStream(plan, st);
-        if (r == CUFFT_SUCCESS)
-            r = cufftExecD2Z(plan, F, reinterpret_cast<cufftDoubleComplex *>(F));
-        e = cudaStreamSynchronize(st);  // the plan's work area outlives the transform
-        cufftDestroy(plan);
-    }
-    if (r != CUFFT_SUCCESS) {
-        *fft_status = (int)r;
-        return cudaErrorUnknown;
-    }
-    if (e != cudaSuccess) return e;
+    cufftResult r = cufftSetWorkArea((cufftHandle)plan.handle, c + out_bytes(p));
+    const size_t field = 2 * (size_t)(p.n[0] / 2 + 1) * p.n[1] * p.n[2];
+    for (int f = 0; f < kSpectraFields && r == CUFFT_SUCCESS; f += plan.batch)
+        r = cufftExecD2Z((cufftHandle)plan.handle, F + f * field,
+                         reinterpret_cast<cufftDoubleComplex *>(F + f * field));
+    *fft_status = (int)r;
+    if (r != CUFFT_SUCCESS) return cudaSuccess;
     // warps per block: as many shell tables as fit 200 KB, at most 8 (a box
     // of 2^31 cells has kmax <= 645)
     const size_t table = sizeof(double) * kSpectra * (size_t)(kmax + 1);
@@ -258,7 +283,7 @@ cudaError_t launch_spectra(const BoxDev &b, void *scratch, double *d_out, int *f
     k_spec_bin<<<kSpecBlocks, 32 * warps, smem, st>>>(reinterpret_cast<const double2 *>(F), p.n[0],
                                                     p.n[1], p.n[2], kmax, partials);
     const int n = kSpectra * kmax;
-    k_spec_reduce<<<(n + 3) / 4, 128, 0, st>>>(partials, kSpecBlocks, n, d_out);
+    k_spec_reduce<<<(n + 3) / 4, 128, 0, st>>>(partials, kSpecBlocks, n, out);
     return cudaGetLastError();
 }
 
