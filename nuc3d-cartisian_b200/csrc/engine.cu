@@ -525,7 +525,9 @@ int Engine::rebuild() {
             if (marched(s, d, mixed)) {
                 march_nmax_[s][d] = std::max(march_nmax_[s][d], p.n[d]);
                 const long long lines = p.N / p.n[d];
-                for (int g = 0; g * 32LL < lines; ++g) march[s][d].push_back({id, g, 0, 0});
+                const int group = d == 0 ? kXLines : kMarchLines;
+                for (int g = 0; (long long)g * group < lines; ++g)
+                    march[s][d].push_back({id, g, 0, 0});
                 continue;
             }
             for (int tc = 0; tc < kInvTileClasses; ++tc) {
@@ -583,7 +585,10 @@ int Engine::rebuild() {
                             cudaMemcpyHostToDevice, stream_));
     ECK(cudaStreamSynchronize(stream_));  // host vectors go out of scope
     ECK(prepare_inviscid_kernels(mixed));
-    if (!mixed) ECK(prepare_march_kernels());
+    if (!mixed) {
+        ECK(prepare_march_kernels());
+        ECK(prepare_xsweep_kernels());
+    }
     ECK(prepare_crweno_kernels(mixed));
     ECK(prepare_stencil_kernels(mixed));
     int per_stage = 0;
@@ -724,6 +729,9 @@ cudaError_t Engine::launch_lines(int d, int in, int prim_mode, cudaStream_t st) 
 template <typename B>
 cudaError_t Engine::launch_sweep(int s, int d, int v, int in, int prim_mode, cudaStream_t st) {
     const Range &m = r_march_[s][d];
+    if (m.n > 0 && d == 0)
+        return launch_xsweep(s, d_boxes_, d_items_ + m.off, m.n, march_nmax_[s][d], in,
+                             kXTiles[v], prim_mode, st);
     if (m.n > 0)
         return launch_march(s, d, d_boxes_, d_items_ + m.off, m.n, march_nmax_[s][d], in,
                             kMarchLen[v], st);

@@ -82,10 +82,10 @@ public:
     // faces per thread and cells per tile of variant v (marched pairs: both are
     // the chunk length)
     int sweep_run(int s, int d, int v) const {
-        return marched(s, d, precision_ == NUC3D_MIXED) ? kMarchLen[v] : kInvRunLen[v];
+        return marched(s, d, precision_ == NUC3D_MIXED) ? march_cells(d, v) : kInvRunLen[v];
     }
     int sweep_tile(int s, int d, int v) const {
-        return marched(s, d, precision_ == NUC3D_MIXED) ? kMarchLen[v] : kInvTileCells[v];
+        return marched(s, d, precision_ == NUC3D_MIXED) ? march_cells(d, v) : kInvTileCells[v];
     }
     // autotuned pencil depth of the 2.5-D stencil kernels: index into
     // kPencilDepths (-1: not tuned yet), the measured milliseconds of one

@@ -762,17 +762,21 @@ cudaError_t launch_inviscid(int scheme, int dir, int variant, const BoxDev *boxe
                             const WorkItem *items, int nitems, int in_slot, int accumulate,
                             int prim_mode, cudaStream_t st) {
     if (nitems <= 0) return cudaSuccess;
-    // (JS and Z along y and z: FP32 only, FP64 marches, see marched())
-    if (scheme == SCHEME_JS && dir == 0) return launch_v<SCHEME_JS, 0, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
-    if (scheme == SCHEME_Z && dir == 0) return launch_v<SCHEME_Z, 0, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+    // (FP32 only: the pairs that march in FP64, see marched())
     if constexpr (sizeof(B) == 4) {
-        if (scheme == SCHEME_JS && dir == 1) return launch_v<SCHEME_JS, 1, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
-        if (scheme == SCHEME_JS) return launch_v<SCHEME_JS, 2, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
-        if (scheme == SCHEME_Z && dir == 1) return launch_v<SCHEME_Z, 1, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
-        if (scheme == SCHEME_Z) return launch_v<SCHEME_Z, 2, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+        if (scheme == SCHEME_JS) {
+            if (dir == 0) return launch_v<SCHEME_JS, 0, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+            if (dir == 1) return launch_v<SCHEME_JS, 1, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+            return launch_v<SCHEME_JS, 2, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+        }
+        if (scheme == SCHEME_Z) {
+            if (dir == 0) return launch_v<SCHEME_Z, 0, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+            if (dir == 1) return launch_v<SCHEME_Z, 1, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+            return launch_v<SCHEME_Z, 2, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+        }
+        if (scheme == SCHEME_W7 && dir == 0) return launch_v<SCHEME_W7, 0, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
     }
-    if (scheme == SCHEME_W7) {
-        if (dir == 0) return launch_v<SCHEME_W7, 0, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
+    if (scheme == SCHEME_W7 && dir > 0) {
         if (dir == 1) return launch_v<SCHEME_W7, 1, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
         return launch_v<SCHEME_W7, 2, B>(variant, boxes, items, nitems, in_slot, accumulate, prim_mode, st);
     }

@@ -150,9 +150,22 @@ cudaError_t launch_inviscid(int scheme, int dir, int variant, const BoxDev *boxe
 // teams, long ones re-read less of the chunk's 6-cell overlap (256^3 z: 8 to
 // 128 cells 0.95, 0.78, 0.67, 0.60, 0.57 ms; 97 x 61 x 45: 22, 20, 22, 26, 26 us).
 constexpr int kMarchLen[kInvVariants] = {8, 16, 32, 64, 128};
+// The FP64 x sweeps of weno5js, weno5z and weno7js (xsweep_kernels.cu): a work
+// item is (box, group of 16 lines), a block walks `tiles` tiles of 32 cells;
+// variant v: kXTiles[v].
+constexpr int kXTiles[kInvVariants] = {1, 2, 4, 8, 16};
+constexpr int kMarchLines = 32, kXLines = 16;
 constexpr bool marched(int scheme, int dir, bool mixed) {
-    return !mixed && dir > 0 && (scheme == SCHEME_JS || scheme == SCHEME_Z);
+    return !mixed && (scheme == SCHEME_JS || scheme == SCHEME_Z ||
+                      (scheme == SCHEME_W7 && dir == 0));
 }
+// cells per work unit of a marched pair's variant
+constexpr int march_cells(int dir, int variant) {
+    return dir == 0 ? 32 * kXTiles[variant] : kMarchLen[variant];
+}
+cudaError_t prepare_xsweep_kernels();
+cudaError_t launch_xsweep(int scheme, const BoxDev *boxes, const WorkItem *items, int nitems,
+                          int nmax, int in_slot, int tiles, int prim_mode, cudaStream_t st);
 cudaError_t prepare_march_kernels();
 cudaError_t launch_march(int scheme, int dir, const BoxDev *boxes, const WorkItem *items,
                          int nitems, int nmax, int in_slot, int len, cudaStream_t st);

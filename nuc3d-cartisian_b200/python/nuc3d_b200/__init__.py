@@ -765,9 +765,10 @@ def _tuning(fn, h, fn_pencil=None, fn_tiles=None):
     """{"<scheme>_<dir>": (chosen "<tile cells>x<run length>", {variant: ms per
     launch}), "pencil_depth": (chosen depth, {depth: ms per viscous-flux +
     update pass})}; the sweep variants are "32x1", "32x2", "32x4", "64x2",
-    "64x4" (cells per tile along the sweep x faces per thread), for the FP64
-    WENO5-JS / WENO5-Z y and z sweeps the marched chunks "8x8", "16x16",
-    "32x32", "64x64", "128x128"."""
+    "64x4" (cells per tile along the sweep x faces per thread); sweeps that
+    march are named by the cells of a chunk, the FP64 WENO5-JS / WENO5-Z y and
+    z sweeps "8x8" to "128x128", the FP64 WENO5 / WENO7 x sweeps "32x32" to
+    "512x512"."""
     import numpy as np
     rl = np.zeros(TUNING_SLOTS, dtype=np.int32)
     ms = np.zeros(3 * TUNING_SLOTS)
@@ -782,7 +783,7 @@ def _tuning(fn, h, fn_pencil=None, fn_tiles=None):
             k = s * 3 + d
             if rl[k] and rl[k] == tc[k]:  # marched chunk
                 times = {f"{L}x{L}": round(float(t), 4) for L, t in
-                         zip((8, 16, 32, 64, 128), [*ms[k * 3:k * 3 + 3], *ms64[k * 2:k * 2 + 2]])}
+                         zip((8, 16, 32, 64, 128) if d else (32, 64, 128, 256, 512), [*ms[k * 3:k * 3 + 3], *ms64[k * 2:k * 2 + 2]])}
                 out[f"{sname}_{dname}"] = (f"{int(tc[k])}x{int(rl[k])}", times)
             elif rl[k]:
                 times = {f"32x{L}": round(float(ms[k * 3 + v]), 4) for v, L in enumerate((1, 2, 4))}
