@@ -364,10 +364,10 @@ __device__ __forceinline__ void line_solve(B *const myF, B *const wA, int ms, in
 
 // Work item (box, a, b, -): DIR 0: lines j = a*TL.., k = b; DIR 1: lines
 // i = a*TL.., k = b; DIR 2: lines i = a*TL.., j = b.
-// prim_mode (x lines only, whose blocks own whole lines): 0 reads the
-// primitives W; 1 first recovers the primitives of the block's lines from
-// the state (prim_cell, k_prim's work, bitwise the same) and writes W; 2
-// also folds their eigenvalues into the box's running maxima.
+// x lines (whose blocks own whole lines) first recover the primitives of the
+// block's lines from the state (prim_cell, k_prim's work, bitwise the same) and
+// write W; prim_mode 2: they also fold their eigenvalues into the box's running
+// maxima.
 template <typename B, int DIR, int SCH>
 __global__ void __launch_bounds__(kCrThreads, sizeof(B) == 8 ? 3 : 4)
     k_crweno_lines(const BoxDev *__restrict__ boxes, const WorkItem *__restrict__ items,
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(kCrThreads, sizeof(B) == 8 ? 3 : 4)
     B *const wA = sRow + (size_t)warp * 3 * ms * 32;  // [j][lane]
     const B inv_d = B(bp.inv_d[DIR]);
 
-    if (DIR == 0 && prim_mode != 0) {  // block-uniform
+    if (DIR == 0) {
         // con2prim of the block's whole lines: the staging below reads their
         // W (written by this block, visible after the barrier)
         const PrimConst pk(bp);

@@ -276,7 +276,6 @@ Engine::~Engine() {
     }
     if (d_boxes_) cudaFreeAsync(d_boxes_, stream_);
     if (d_items_) cudaFreeAsync(d_items_, stream_);
-    if (d_rhs_ptrs_) cudaFreeAsync(d_rhs_ptrs_, stream_);
     if (d_stats_) cudaFreeAsync(d_stats_, stream_);
     cudaStreamSynchronize(stream_);
     spectra_plan_.release();
@@ -567,10 +566,8 @@ int Engine::rebuild() {
         for (int d = 0; d < 3; ++d) append(cr[c][d], r_cr_[c][d]);
     if ((int)boxes_.size() > d_boxes_cap_) {
         if (d_boxes_) ECK(cudaFreeAsync(d_boxes_, stream_));
-        if (d_rhs_ptrs_) ECK(cudaFreeAsync(d_rhs_ptrs_, stream_));
         d_boxes_cap_ = std::max<int>(8, (int)boxes_.size() * 2);
         ECK(device_alloc(&d_boxes_, sizeof(BoxDev) * d_boxes_cap_));
-        ECK(device_alloc(&d_rhs_ptrs_, sizeof(double *) * 5 * d_boxes_cap_));
     }
     if (all.size() > d_items_cap_) {
         if (d_items_) ECK(cudaFreeAsync(d_items_, stream_));
@@ -702,7 +699,7 @@ int Engine::enqueue_step_t(cudaStream_t st) {
         if (fork) ECK(cudaStreamWaitEvent(st, fork_ev_[1], 0));
         {
             ProfScope ps(this, NUC3D_PROF_UPDATE);
-            StageArgs sa{stage, in, out, nullptr};
+            StageArgs sa{stage, in, out};
             ECK(launch_update_classes<B>(pv(), sa, st));
         }
     }
@@ -844,7 +841,7 @@ int Engine::autotune() {
     }
     invalidate_graph();
     if (!need_sweep && !tune_pencil) return NUC3D_OK;
-    ECK(launch_prim(d_boxes_, d_items_ + r_prim_.off, r_prim_.n, 0, 0, stream_));
+    ECK(launch_prim(d_boxes_, d_items_ + r_prim_.off, r_prim_.n, 0, stream_));
     cudaEvent_t e0, e1;
     ECK(cudaEventCreate(&e0));
     ECK(cudaEventCreate(&e1));
@@ -901,7 +898,7 @@ int Engine::autotune() {
                 pencil_tune_ms[v] = 0.0;
                 continue;
             }
-            const StageArgs sa{0, 0, 1, nullptr};
+            const StageArgs sa{0, 0, 1};
             const double ms = time3([&]() {
                 cudaError_t err = cudaSuccess;
                 if (any_visc_)
@@ -996,26 +993,23 @@ int Engine::history(int id, int n, double *h_dt, double *h_res) {
     return NUC3D_OK;
 }
 
+// One RHS evaluation as a step's first stage runs it: the x sweep recovers the
+// primitives and folds the eigenvalue maxima; the update writes to d_rhs.
 template <typename B>
-int Engine::enqueue_rhs_t(int id, double *const d_rhs[5]) {
+int Engine::enqueue_rhs_t(double *const d_rhs[5]) {
     const int nb = (int)boxes_.size();
-    const WorkItem *it = d_items_;
-    double *ptrs[5];
-    for (int e = 0; e < 5; ++e) ptrs[e] = d_rhs[e];
-    ECK(cudaMemcpyAsync(d_rhs_ptrs_ + 5 * id, ptrs, sizeof ptrs, cudaMemcpyHostToDevice, stream_));
     ECK(launch_clear_eig(d_boxes_, nb, stream_));
-    ECK(launch_prim(d_boxes_, it + r_prim_.off, r_prim_.n, 0, 1, stream_));
-    ECK(launch_dt(d_boxes_, nb, stream_));
     for (int d = 0; d < 3; ++d) {
         for (int s = 0; s < kSchemes; ++s)
-            ECK((launch_sweep<B>(s, d, inv_variant[s][d], 0, 0, stream_)));
-        ECK(launch_lines<B>(d, 0, 0, stream_));
+            ECK((launch_sweep<B>(s, d, inv_variant[s][d], 0, d == 0 ? 2 : 0, stream_)));
+        ECK(launch_lines<B>(d, 0, d == 0 ? 2 : 0, stream_));
+        if (d == 0) ECK(launch_dt(d_boxes_, nb, stream_));
     }
     if (any_visc_) ECK(launch_visc_classes<B>(pv(), stream_));
     ECK(enqueue_forcing<B>(stream_));
-    StageArgs sa{-1, 0, 0, d_rhs_ptrs_};
+    StageArgs sa{-1, 0, 0};
+    for (int e = 0; e < 5; ++e) sa.rhs_out[e] = d_rhs[e];
     ECK(launch_update_classes<B>(pv(), sa, stream_));
-    ECK(cudaStreamSynchronize(stream_));  // ptrs is a host stack array
     return NUC3D_OK;
 }
 
@@ -1033,13 +1027,12 @@ int Engine::rhs(int id, double *const d_rhs[5], double *h_dt_local) {
         int rc = autotune();
         if (rc) return rc;
     }
-    int rc = precision_ == NUC3D_MIXED ? enqueue_rhs_t<float>(id, d_rhs) : enqueue_rhs_t<double>(id, d_rhs);
+    int rc = precision_ == NUC3D_MIXED ? enqueue_rhs_t<float>(d_rhs) : enqueue_rhs_t<double>(d_rhs);
     if (rc) return rc;
-    if (h_dt_local) {
+    if (h_dt_local)
         ECK(cudaMemcpyAsync(h_dt_local, &boxes_[id].dev.sc->dt_local, sizeof(double),
                             cudaMemcpyDeviceToHost, stream_));
-        ECK(cudaStreamSynchronize(stream_));
-    }
+    ECK(cudaStreamSynchronize(stream_));
     return NUC3D_OK;
 }
 
@@ -1119,7 +1112,7 @@ int Engine::stats(int id, double out[26]) {
     if (!b.dev.active) return set_last_error(NUC3D_ERR_INVALID, "box is not active");
     if (!d_stats_) ECK(device_alloc(&d_stats_, sizeof(double) * stats_scratch_doubles()));
     // primitives of U[0] into W (scratch between steps), then the sums
-    ECK(launch_prim(d_boxes_, d_items_ + r_prim_.off + b.prim_off, b.prim_n, 0, 0, stream_));
+    ECK(launch_prim(d_boxes_, d_items_ + r_prim_.off + b.prim_off, b.prim_n, 0, stream_));
     ECK(launch_stats(b.dev, d_stats_, stream_));
     double sums[kStatsSums];
     ECK(cudaMemcpyAsync(sums, d_stats_, sizeof sums, cudaMemcpyDeviceToHost, stream_));
@@ -1151,7 +1144,7 @@ int Engine::spectra(int id, double *out, int *kmax_out) {
             cudaGetLastError();
             return set_last_error(NUC3D_ERR_NOMEM, "no device memory for the spectra scratch");
         }
-        e = launch_prim(d_boxes_, d_items_ + r_prim_.off + b.prim_off, b.prim_n, 0, 0, stream_);
+        e = launch_prim(d_boxes_, d_items_ + r_prim_.off + b.prim_off, b.prim_n, 0, stream_);
         double *d_out = nullptr;
         if (e == cudaSuccess)
             e = launch_spectra(b.dev, spectra_plan_, scratch, &d_out, &fft_status, stream_);

@@ -20,15 +20,13 @@ namespace nuc3d {
 
 // A work item is (box, first cell chunk, cell count).
 __global__ void __launch_bounds__(256, 4) k_prim(const BoxDev *__restrict__ boxes,
-                                                 const WorkItem *__restrict__ items, int in_slot,
-                                                 int want_eig) {
+                                                 const WorkItem *__restrict__ items, int in_slot) {
     const WorkItem it = items[blockIdx.x];
     const BoxDev &bd = boxes[it.box];
     if (!bd.active) return;
     const long long np = bd.np;
     const double *__restrict__ q = fieldU(bd, in_slot, 0);
     const PrimConst pk(bd.p);
-    double lx = 0.0, ly = 0.0, lz = 0.0;
     const long long n0 = (long long)it.a * kPrimChunk, n1 = n0 + it.b;
     // the next cell's state is loaded while the current one is converted
     long long n = n0 + threadIdx.x;
@@ -47,12 +45,7 @@ __global__ void __launch_bounds__(256, 4) k_prim(const BoxDev *__restrict__ boxe
         PrimCell o;
         prim_cell(pk, Q, o);
         prim_store(bd, n, o);
-        lx = fmax(add_(fabs(o.u), o.c), lx);
-        ly = fmax(add_(fabs(o.v), o.c), ly);
-        lz = fmax(add_(fabs(o.w), o.c), lz);
     }
-    if (!want_eig) return;
-    eig_block_max(bd, lx, ly, lz);
 }
 
 __global__ void k_clear_eig(const BoxDev *boxes, int nboxes) {
@@ -220,10 +213,10 @@ __device__ __forceinline__ void inviscid_body(const BoxDev *__restrict__ boxes,
         return a + sy * fixed + sz * pos;
     };
     const int riemann = bp.riemann;
-    // prim_mode (x sweep only): 0 reads u_n, p, c from W; 1 recovers the
-    // primitives from the state (prim_cell) and writes W for the tile's own
-    // cells; 2 also folds their eigenvalues into the box's maxima
-    const bool own_prim = DIR == 0 && prim_mode != 0;
+    // the x sweep recovers the primitives from the state (prim_cell) and writes
+    // W for the tile's own cells; prim_mode 2 also folds their eigenvalues into
+    // the box's maxima
+    constexpr bool own_prim = DIR == 0;
     const PrimConst pk(bp);
     double eg[3] = {0.0, 0.0, 0.0};
     // split fluxes of cell g; store: g is one of the tile's own cells
@@ -837,9 +830,9 @@ cudaError_t prepare_inviscid_kernels(bool mixed) {
 }
 
 cudaError_t launch_prim(const BoxDev *boxes, const WorkItem *items, int nitems, int in_slot,
-                        int want_eig, cudaStream_t st) {
+                        cudaStream_t st) {
     if (nitems <= 0) return cudaSuccess;
-    k_prim<<<nitems, 256, 0, st>>>(boxes, items, in_slot, want_eig);
+    k_prim<<<nitems, 256, 0, st>>>(boxes, items, in_slot);
     return cudaGetLastError();
 }
 

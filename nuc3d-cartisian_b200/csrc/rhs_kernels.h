@@ -84,12 +84,13 @@ struct WorkItem {
 };
 
 // Stage addressing: which U buffers are input/output of RK stage `stage`;
-// stage -1 evaluates the RHS of U[0] and writes it to `rhs_out`.
+// stage -1 evaluates the RHS of U[0] of the one active box and writes it to
+// `rhs_out`.
 struct StageArgs {
     int stage;
     int in_slot;             // U index read by the RHS (0, 1, 2)
     int out_slot;            // U index written by the update (1, 2, 0)
-    double *const *rhs_out;  // device array of 5 pointers per box (stage -1 only)
+    double *rhs_out[5];      // (stage -1 only)
 };
 
 // Tile geometry of the batched kernels (host and device agree on these).
@@ -111,7 +112,7 @@ constexpr int kPrimChunk = 4096;                  // cells per k_prim work item
 // memory size (once per device, before any launch or stream capture).
 cudaError_t prepare_inviscid_kernels(bool mixed);
 cudaError_t launch_prim(const BoxDev *boxes, const WorkItem *items, int nitems, int in_slot,
-                        int want_eig, cudaStream_t st);
+                        cudaStream_t st);
 cudaError_t launch_dt(const BoxDev *boxes, int nboxes, cudaStream_t st);
 cudaError_t launch_residual(const BoxDev *boxes, int nboxes, cudaStream_t st);
 cudaError_t launch_clear_eig(const BoxDev *boxes, int nboxes, cudaStream_t st);
@@ -134,10 +135,9 @@ constexpr int kLineScheme[kLineSchemes] = {SCHEME_CR, SCHEME_HC, SCHEME_H77};
 constexpr int line_slot(int scheme) {
     return scheme == SCHEME_CR ? 0 : (scheme == SCHEME_HC ? 1 : (scheme == SCHEME_H77 ? 2 : -1));
 }
-// prim_mode (x sweep only): 0 reads the primitives W; 1 recovers them from
-// the state while staging and writes W for the tile's own cells (k_prim's
-// work, bitwise the same); 2 also folds their eigenvalues into the boxes'
-// running maxima (k_prim with want_eig)
+// The x sweep recovers the primitives from the state while staging and writes W
+// for the tile's own cells (k_prim's work, bitwise the same); prim_mode 2: it
+// also folds their eigenvalues into the boxes' running maxima (1: not)
 template <typename B>
 cudaError_t launch_inviscid(int scheme, int dir, int variant, const BoxDev *boxes,
                             const WorkItem *items, int nitems, int in_slot, int accumulate,

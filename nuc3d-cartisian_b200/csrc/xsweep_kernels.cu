@@ -141,8 +141,8 @@ struct XGeom {
 }  // namespace
 
 // Work item (box, group of 16 lines); blockIdx.y: the chunk of `tiles` tiles.
-// PM 0: u_n, p, c from W; 1: recovered from the state, W written for the
-// tile's own cells; 2: their eigenvalues folded into the box's maxima as well.
+// The primitives are recovered from the state and W is written for the tile's
+// own cells; PM 2: their eigenvalues are folded into the box's maxima as well.
 template <int SCHEME, int PM>
 __global__ void __launch_bounds__(kThreads, SCHEME == SCHEME_W7 ? 3 : 4)
     k_xsweep(const BoxDev *__restrict__ boxes, const WorkItem *__restrict__ items, int in_slot,
@@ -191,26 +191,17 @@ __global__ void __launch_bounds__(kThreads, SCHEME == SCHEME_W7 ? 3 : 4)
             double q[5];
 #pragma unroll
             for (int v = 0; v < 5; ++v) q[v] = qbase[v * np + g];
-            double un, pr, c;
-            if (PM) {
-                PrimCell o;
-                prim_cell(pk, q, o);
-                un = o.u;
-                pr = o.p;
-                c = o.c;
-                if (own) {
-                    prim_store(bd, g, o);
-                    if (PM == 2) {
-                        eg[0] = fmax(add_(fabs(o.u), o.c), eg[0]);
-                        eg[1] = fmax(add_(fabs(o.v), o.c), eg[1]);
-                        eg[2] = fmax(add_(fabs(o.w), o.c), eg[2]);
-                    }
+            PrimCell o;
+            prim_cell(pk, q, o);
+            if (own) {
+                prim_store(bd, g, o);
+                if (PM == 2) {
+                    eg[0] = fmax(add_(fabs(o.u), o.c), eg[0]);
+                    eg[1] = fmax(add_(fabs(o.v), o.c), eg[1]);
+                    eg[2] = fmax(add_(fabs(o.w), o.c), eg[2]);
                 }
-            } else {
-                un = fieldW(bd, 0)[g];
-                pr = fieldW(bd, 3)[g];
-                c = fieldW(bd, 4)[g];
             }
+            const double un = o.u, pr = o.p, c = o.c;
             if (!W7 && riemann == RIEMANN_LF) {  // block-uniform
 #pragma unroll
                 for (int v = 0; v < 5; ++v) {
@@ -287,9 +278,7 @@ namespace {
 using XSweep = void (*)(const BoxDev *, const WorkItem *, int, int);
 template <int SCHEME>
 XSweep xsweep_pm(int prim_mode) {
-    return prim_mode == 0   ? k_xsweep<SCHEME, 0>
-           : prim_mode == 1 ? k_xsweep<SCHEME, 1>
-                            : k_xsweep<SCHEME, 2>;
+    return prim_mode == 2 ? k_xsweep<SCHEME, 2> : k_xsweep<SCHEME, 1>;
 }
 XSweep xsweep_kernel(int scheme, int prim_mode, size_t &smem) {
     smem = scheme == SCHEME_W7  ? XGeom<SCHEME_W7>::SMEM
@@ -303,7 +292,7 @@ XSweep xsweep_kernel(int scheme, int prim_mode, size_t &smem) {
 
 cudaError_t prepare_xsweep_kernels() {
     for (int s : {SCHEME_JS, SCHEME_Z, SCHEME_W7})
-        for (int m = 0; m < 3; ++m) {
+        for (int m = 1; m < 3; ++m) {
             size_t smem;
             const XSweep k = xsweep_kernel(s, m, smem);
             cudaError_t e =
