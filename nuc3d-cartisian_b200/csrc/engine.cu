@@ -276,6 +276,7 @@ Engine::~Engine() {
     }
     if (d_boxes_) cudaFreeAsync(d_boxes_, stream_);
     if (d_items_) cudaFreeAsync(d_items_, stream_);
+    if (d_rhs_ptrs_) cudaFreeAsync(d_rhs_ptrs_, stream_);
     if (d_stats_) cudaFreeAsync(d_stats_, stream_);
     cudaStreamSynchronize(stream_);
     spectra_plan_.release();
@@ -566,8 +567,10 @@ int Engine::rebuild() {
         for (int d = 0; d < 3; ++d) append(cr[c][d], r_cr_[c][d]);
     if ((int)boxes_.size() > d_boxes_cap_) {
         if (d_boxes_) ECK(cudaFreeAsync(d_boxes_, stream_));
+        if (d_rhs_ptrs_) ECK(cudaFreeAsync(d_rhs_ptrs_, stream_));
         d_boxes_cap_ = std::max<int>(8, (int)boxes_.size() * 2);
         ECK(device_alloc(&d_boxes_, sizeof(BoxDev) * d_boxes_cap_));
+        ECK(device_alloc(&d_rhs_ptrs_, sizeof(double *) * 5 * d_boxes_cap_));
     }
     if (all.size() > d_items_cap_) {
         if (d_items_) ECK(cudaFreeAsync(d_items_, stream_));
@@ -699,7 +702,7 @@ int Engine::enqueue_step_t(cudaStream_t st) {
         if (fork) ECK(cudaStreamWaitEvent(st, fork_ev_[1], 0));
         {
             ProfScope ps(this, NUC3D_PROF_UPDATE);
-            StageArgs sa{stage, in, out};
+            StageArgs sa{stage, in, out, nullptr};
             ECK(launch_update_classes<B>(pv(), sa, st));
         }
     }
@@ -898,7 +901,7 @@ int Engine::autotune() {
                 pencil_tune_ms[v] = 0.0;
                 continue;
             }
-            const StageArgs sa{0, 0, 1};
+            const StageArgs sa{0, 0, 1, nullptr};
             const double ms = time3([&]() {
                 cudaError_t err = cudaSuccess;
                 if (any_visc_)
@@ -995,9 +998,15 @@ int Engine::history(int id, int n, double *h_dt, double *h_res) {
 
 // One RHS evaluation as a step's first stage runs it: the x sweep recovers the
 // primitives and folds the eigenvalue maxima; the update writes to d_rhs.
+// (The copy from pageable memory has read ptrs when it returns.  The five
+// pointers by value in StageArgs cost the update kernel registers: 0.27 -> 0.31
+// ms per step of a 192 x 96 x 80 box.)
 template <typename B>
-int Engine::enqueue_rhs_t(double *const d_rhs[5]) {
+int Engine::enqueue_rhs_t(int id, double *const d_rhs[5]) {
     const int nb = (int)boxes_.size();
+    double *ptrs[5];
+    for (int e = 0; e < 5; ++e) ptrs[e] = d_rhs[e];
+    ECK(cudaMemcpyAsync(d_rhs_ptrs_ + 5 * id, ptrs, sizeof ptrs, cudaMemcpyHostToDevice, stream_));
     ECK(launch_clear_eig(d_boxes_, nb, stream_));
     for (int d = 0; d < 3; ++d) {
         for (int s = 0; s < kSchemes; ++s)
@@ -1007,8 +1016,7 @@ int Engine::enqueue_rhs_t(double *const d_rhs[5]) {
     }
     if (any_visc_) ECK(launch_visc_classes<B>(pv(), stream_));
     ECK(enqueue_forcing<B>(stream_));
-    StageArgs sa{-1, 0, 0};
-    for (int e = 0; e < 5; ++e) sa.rhs_out[e] = d_rhs[e];
+    StageArgs sa{-1, 0, 0, d_rhs_ptrs_};
     ECK(launch_update_classes<B>(pv(), sa, stream_));
     return NUC3D_OK;
 }
@@ -1027,7 +1035,7 @@ int Engine::rhs(int id, double *const d_rhs[5], double *h_dt_local) {
         int rc = autotune();
         if (rc) return rc;
     }
-    int rc = precision_ == NUC3D_MIXED ? enqueue_rhs_t<float>(d_rhs) : enqueue_rhs_t<double>(d_rhs);
+    int rc = precision_ == NUC3D_MIXED ? enqueue_rhs_t<float>(id, d_rhs) : enqueue_rhs_t<double>(id, d_rhs);
     if (rc) return rc;
     if (h_dt_local)
         ECK(cudaMemcpyAsync(h_dt_local, &boxes_[id].dev.sc->dt_local, sizeof(double),

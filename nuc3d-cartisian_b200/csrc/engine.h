@@ -112,7 +112,7 @@ private:
     template <typename B>
     int enqueue_step_t(cudaStream_t s);
     template <typename B>
-    int enqueue_rhs_t(double *const d_rhs[5]);
+    int enqueue_rhs_t(int id, double *const d_rhs[5]);
     template <typename B>
     cudaError_t enqueue_forcing(cudaStream_t st);
     // the 2.5-D kernels of both stencil classes at pencil-depth variant v
@@ -200,6 +200,7 @@ private:
     int h_flags_cap_ = 0;
     int device_ = 0;                      // the device current at construction
     cudaEvent_t copy_ev_[2] = {nullptr, nullptr};  // this engine's last upload / download
+    double **d_rhs_ptrs_ = nullptr;  // 5 per box, for stage -1
     double *d_stats_ = nullptr;       // statistics scratch
     // profiling events
     std::vector<cudaEvent_t> ev_pool_;

@@ -84,13 +84,12 @@ struct WorkItem {
 };
 
 // Stage addressing: which U buffers are input/output of RK stage `stage`;
-// stage -1 evaluates the RHS of U[0] of the one active box and writes it to
-// `rhs_out`.
+// stage -1 evaluates the RHS of U[0] and writes it to `rhs_out`.
 struct StageArgs {
     int stage;
     int in_slot;             // U index read by the RHS (0, 1, 2)
     int out_slot;            // U index written by the update (1, 2, 0)
-    double *rhs_out[5];      // (stage -1 only)
+    double *const *rhs_out;  // device array of 5 pointers per box (stage -1 only)
 };
 
 // Tile geometry of the batched kernels (host and device agree on these).

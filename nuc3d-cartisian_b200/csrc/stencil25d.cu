@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(TX *TY, 2)
             }
             if (stage < 0) {
 #pragma unroll
-                for (int e = 0; e < 5; ++e) sa.rhs_out[e][g] = double(Rv[e]);
+                for (int e = 0; e < 5; ++e) sa.rhs_out[5 * it.box + e][g] = double(Rv[e]);
             } else {
 #pragma unroll
                 for (int e = 0; e < 5; ++e) {
