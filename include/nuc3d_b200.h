@@ -280,7 +280,12 @@ NUC3D_API int nuc3d_probe_peak(int precision, double *tflops);
  * only, because its FP32 staging is offset by each line's value at the
  * tile's first cell and another tile length would round differently);
  * NUC3D_TUNING_SLOTS ints and 2*NUC3D_TUNING_SLOTS doubles, either may be
- * NULL. */
+ * NULL.
+ * In double precision weno5js and weno5z (x, y, z) and weno7js (x) sweep by
+ * walking a line in chunks instead: their five variants are the chunk lengths
+ * in cells (y, z: 8, 16, 32, 64, 128; x: 32, 64, 128, 256, 512), reported as
+ * both run_len and tile_cells, the milliseconds in the same order in ms (the
+ * first three) and ms64 (the last two). */
 #define NUC3D_TUNING_SLOTS 27
 NUC3D_API int nuc3d_tuning(const nuc3d_ctx *ctx, int *run_len, double *ms);
 NUC3D_API int nuc3d_batch_tuning(const nuc3d_batch *b, int *run_len, double *ms);
@@ -291,10 +296,11 @@ NUC3D_API int nuc3d_batch_tuning_tiles(const nuc3d_batch *b, int *tile_cells, do
  * marches (each tile re-reads a 6-plane halo, so deeper pencils read less but
  * make fewer, longer blocks).  The first step, and every step after the
  * batch's active cells have grown or shrunk past a factor 2 of those it was
- * tuned at, times one viscous-flux + update pass at each of
- * NUC3D_PENCIL_DEPTHS depths on the live boxes and keeps the fastest.
- * *depth receives the chosen depth (0 = not tuned), ms (3 doubles, may be
- * NULL) the measured milliseconds per pass for depths {32, 16, 64}. */
+ * tuned at into a size not tuned before, times viscous-flux + update passes
+ * on the live boxes and keeps the fastest depth; boxes too small to fill the
+ * GPU may get 8, 4 or 2 planes.  *depth receives the chosen depth (0 = not
+ * tuned), ms (NUC3D_PENCIL_DEPTHS doubles, may be NULL) the measured
+ * milliseconds per pass for depths {32, 16, 64}. */
 #define NUC3D_PENCIL_DEPTHS 3
 NUC3D_API int nuc3d_tuning_pencil(const nuc3d_ctx *ctx, int *depth, double *ms);
 NUC3D_API int nuc3d_batch_tuning_pencil(const nuc3d_batch *b, int *depth, double *ms);

@@ -12,7 +12,7 @@
 // Bound: the FP64 pipe (about 86 FP64 instructions per cell and equation, 158
 // instructions in all).  A march forms each difference, square and split once
 // per cell: a tile of 32 cells whose threads each hold a run of 2 or 4 faces
-// (k_inviscid, the sweep of the other schemes and directions) rebuilds its
+// (k_inviscid, which these sweeps replaced) rebuilds its
 // windows for every run and stages 38 cells for 32.  256^3 WENO5-Z, per launch:
 // y 0.68 -> 0.59 ms, z 0.70 -> 0.57 ms (about 3/4 of the FP64 pipe's rate).
 // Measured beside it: one warp per sign (30 warps of 64 registers) 0.89 / 0.88,
@@ -20,7 +20,7 @@
 // the loads a cell ahead in registers 0.70 / 0.70, with the double buffer 0.67.
 // Along x the lanes' lines run along the fastest axis and the same march
 // behind a transposing staging pass took 0.91-1.05 ms against the tiles' 0.83,
-// so x keeps the tiles.
+// so x walks tiles (xsweep_kernels.cu).
 //
 // Window: when cell p arrives both signs hold the cells p-4..p.  With f2 the
 // value of cell p-2 that is the '+' stencil of face p-1 and, mirrored, the

@@ -249,7 +249,7 @@ __device__ __forceinline__ float weno_z_combine(float is0, float is1, float is2,
     return mul_(fma_(a2, q2, fma_(a1, q1, mul_(a0, q0))), frcp_fast(add_(add_(a0, a1), a2)));
 }
 
-// The same combinations in offset form for the sweeps: with dq_k = q_k - f2
+// The same combinations in offset form for the FP32 sweeps: with dq_k = q_k - f2
 // the face is f2 + sum(w_k dq_k) / sum(w_k), which saves the candidates'
 // common part and keeps the rounding relative to the local variation.  The
 // linear weights are 0.1 (1, 6, 3); the 0.1 cancels in the ratio and the 6
@@ -257,21 +257,7 @@ __device__ __forceinline__ float weno_z_combine(float is0, float is1, float is2,
 // and the face is f2 + (w0 g0 + w1 g1 + w2 g2) / (w0 + 6 w1 + 3 w2) with w_k
 // the weights without their linear factor.  The indicators arrive scaled by
 // 4 (is_k = 4 beta_k, see weno5_face_dq) and eps with them, an exact scaling
-// that leaves every weight ratio bitwise unchanged.  WENO5-Z's
-// (beta + 1e-40)^2 is formed as beta^2 + 1e-80 (the cross term is below
-// 1e-40 of beta).
-__device__ __forceinline__ double weno_js_combine_dq(double is0, double is1, double is2,
-                                                     double g0, double g1, double g2,
-                                                     double f2) {
-    const double ss = 4.0 * 1.0e-6;  // 4 eps
-    double s0 = add_(ss, is0), s1 = add_(ss, is1), s2 = add_(ss, is2);
-    s0 = mul_(s0, s0);
-    s1 = mul_(s1, s1);
-    s2 = mul_(s2, s2);
-    const double w0 = mul_(s1, s2), w1 = mul_(s0, s2), w2 = mul_(s0, s1);
-    return fma_(fma_(w2, g2, fma_(w1, g1, mul_(w0, g0))),
-                drcp_nr(fma_(6.0, w1, fma_(3.0, w2, w0))), f2);
-}
+// that leaves every weight ratio bitwise unchanged.
 __device__ __forceinline__ float weno_js_combine_dq(float is0, float is1, float is2, float g0,
                                                     float g1, float g2, float f2) {
     const float ss = 4.0f * 1.0e-6f;  // 4 eps
@@ -279,22 +265,6 @@ __device__ __forceinline__ float weno_js_combine_dq(float is0, float is1, float 
     const float a0 = mul_(r0, r0), a1 = mul_(r1, r1), a2 = mul_(r2, r2);
     return fma_(fma_(a2, g2, fma_(a1, g1, mul_(a0, g0))),
                 frcp_fast(fma_(6.0f, a1, fma_(3.0f, a2, a0))), f2);
-}
-__device__ __forceinline__ double weno_z_combine_dq(double is0, double is1, double is2,
-                                                    double g0, double g1, double g2,
-                                                    double f2) {
-    const double ss2 = 16.0 * 1.0e-80;  // (4 eps)^2, eps = 1e-40
-    const double tau = sub_(is2, is0);
-    const double t2 = mul_(tau, tau);
-    double s0 = fma_(is0, is0, ss2), s1 = fma_(is1, is1, ss2), s2 = fma_(is2, is2, ss2);
-    // alpha_k / c_k * s0^2 s1^2 s2^2 = (s_k^2 + tau^2) prod_{j!=k} s_j^2
-    //                                = P + tau^2 prod_{j!=k} s_j^2,  P = s0^2 s1^2 s2^2
-    // (three products, one more for P, three FMAs)
-    const double p12 = mul_(s1, s2), p02 = mul_(s0, s2), p01 = mul_(s0, s1);
-    const double P = mul_(s0, p12);
-    const double w0 = fma_(t2, p12, P), w1 = fma_(t2, p02, P), w2 = fma_(t2, p01, P);
-    return fma_(fma_(w2, g2, fma_(w1, g1, mul_(w0, g0))),
-                drcp_nr(fma_(6.0, w1, fma_(3.0, w2, w0))), f2);
 }
 __device__ __forceinline__ float weno_z_combine_dq(float is0, float is1, float is2, float g0,
                                                    float g1, float g2, float f2) {
@@ -317,23 +287,23 @@ __device__ __forceinline__ float weno_z_combine_dq(float is0, float is1, float i
 //   E2 = D2 - 2 a32,   4 beta_k = dd_k + E_k^2,  dd_k = 4 (13/12) D_k^2,
 // and the candidates (schemes.hpp:14-18) as f2 + dq_k:
 //   dq0 = D0/3 + a21/2,  6 dq1 = a21 + 2 a32,  3 dq2 = 2 a32 - a43/2.
-template <int SCHEME, typename B>
-__device__ __forceinline__ B weno5_face_dq(B f2, B a21, B a32, B a43, B D0, B D2, B dd0, B dd1,
-                                           B dd2) {
-    const B h = B(0.5);
-    const B e0 = fma_(B(2), a21, D0);
-    const B e1 = add_(a21, a32);
-    const B e2 = fma_(B(-2), a32, D2);
-    const B is0 = fma_(e0, e0, dd0), is1 = fma_(e1, e1, dd1), is2 = fma_(e2, e2, dd2);
-    const B g0 = fma_(B(1.0 / 3.0), D0, mul_(h, a21));
-    const B g1 = fma_(B(2), a32, a21);
-    const B g2 = fma_(B(2), a32, mul_(B(-0.5), a43));
+template <int SCHEME>
+__device__ __forceinline__ float weno5_face_dq(float f2, float a21, float a32, float a43, float D0, float D2, float dd0, float dd1,
+                                           float dd2) {
+    const float h = 0.5f;
+    const float e0 = fma_(2.0f, a21, D0);
+    const float e1 = add_(a21, a32);
+    const float e2 = fma_(-2.0f, a32, D2);
+    const float is0 = fma_(e0, e0, dd0), is1 = fma_(e1, e1, dd1), is2 = fma_(e2, e2, dd2);
+    const float g0 = fma_(float(1.0 / 3.0), D0, mul_(h, a21));
+    const float g1 = fma_(2.0f, a32, a21);
+    const float g2 = fma_(2.0f, a32, mul_(-0.5f, a43));
     if (SCHEME == SCHEME_Z) return weno_z_combine_dq(is0, is1, is2, g0, g1, g2, f2);
     return weno_js_combine_dq(is0, is1, is2, g0, g1, g2, f2);
 }
 
 // Two FP32 faces at once (component x: one stencil, y: another), packed:
-// component-wise the operations of weno5_face_dq<SCHEME, float> with
+// component-wise the operations of weno5_face_dq<SCHEME> with
 // weno_z_combine_dq / weno_js_combine_dq, in the same order, so each
 // component is bitwise that face.  The reciprocals, |.| and min stay scalar.
 template <int SCHEME>
@@ -1003,23 +973,8 @@ struct DiffAt {
     }
 };
 
-// Viscosity and heat-conduction coefficient (physicsModel.cpp:193-266).
-template <typename B>
-__device__ __forceinline__ void viscosity(const BoxParams &bp, B T, B &miu, B &coeff) {
-    B m;
-    if (bp.visc_model == VISC_SUTHERLAND) {
-        B tr = B(bp.tref_nd);
-        m = (B(1) + tr) / (T + tr) * (T * sqrt(T)) / B(bp.reynolds);
-    } else if (bp.visc_model == VISC_CONSTANT) {
-        m = B(1) / B(bp.reynolds);
-    } else {
-        m = pow(T, B(bp.powerlaw_exp)) / B(bp.reynolds);
-    }
-    miu = m;
-    coeff = m / B((bp.gamma - 1.0) * bp.mach * bp.mach * bp.prandtl);
-}
-
-// The same coefficients with the box's constants formed once per block:
+// Viscosity and heat-conduction coefficient (physicsModel.cpp:193-266) with the
+// box's constants formed once per block:
 // Sutherland as ((1 + Tref)/Re) T sqrt(T) / (T + Tref) with one correctly
 // rounded reciprocal, and the divisions by Re and by (gamma-1) M^2 Pr as
 // multiplications by their reciprocals (each within an ulp or two of the

@@ -1,11 +1,12 @@
 // Batched whole-box kernels: primitive recovery, dt, residual and the
 // directional WENO5 / WENO7 sweeps.
 //
-// One RK stage = k_inviscid<x> (which recovers the primitives of its tiles:
-// k_prim's work; k_prim itself runs first for boxes whose x lines use the
-// line kernel) -> [k_dt on the first stage] -> [k_visc_flux25] ->
-// k_inviscid<y> -> k_inviscid<z> -> k_update25, each one launch for every
-// box of a batch.
+// One RK stage = x sweep (which recovers the primitives of its tiles: k_prim's
+// work) -> [k_dt on the first stage] -> [k_visc_flux25] -> y sweep -> z sweep ->
+// k_update25, each one launch for every box of a batch.  The tiled sweeps here
+// serve the mixed precision and, in FP64, weno7js along y and z, hccs78, weno3js
+// and upwind1st; the other FP64 sweeps: march_kernels.cu, xsweep_kernels.cu and
+// thomas_kernels.cu, the line solves: crweno_kernels.cu.
 // The reference's per-direction rotated copies, halo buffers and MPI
 // self-messages (euler3d.cpp:307-387, NaiverStokes3d.cpp:87-369,
 // MPICommunicator.cpp:81-132) become periodic index wraps in the tile loads.
@@ -445,218 +446,136 @@ __device__ __forceinline__ void inviscid_body(const BoxDev *__restrict__ boxes,
                                               sF[G::sf(5 + e, l, m + 2)],
                                               sF[G::sf(5 + e, l, m + 1)]));
             }
+        } else if constexpr (DIR == 0) {
+            // WENO5 (FP32 only: the FP64 pairs march, see marched()).
+            // FP32 x sweep: faces in pairs on the packed f32x2 arithmetic.  The
+            // thread's K faces (R, and the next run's first on the last
+            // run) are taken '+' in ascending order beside '-' in
+            // descending order: the '+' stencil of face m0+j (positions
+            // m..m+4) and the '-' stencil of face m0+K-1-j (positions
+            // m'+5..m'+1) both step by dropping f0 and gaining a new f4,
+            // so one packed window (component x: '+', y: '-') carries
+            // both.  Component-wise the operations are those of the
+            // one-sided windows below, so every face is bitwise the same.
+            // (256^3 mixed step, x sweeps: WENO5-Z 1.895 -> 1.84 ms, WENO5-JS
+            // 1.81 -> 1.75 ms.  The y/z sweeps wait on their staging loads,
+            // not on FP32 issue: there the packed form measured the same
+            // (WENO5-Z) or 2-4 % slower (WENO5-JS), so they keep the
+            // one-sided form.)
+            const int K = R + (last ? 1 : 0);
+            const int mq = m0 + K - 1;  // the '-' side's first face
+            const int vp = e, vm = 5 + e;
+            float2 w0 = make_float2(sF[G::sf(vp, l, m0)], sF[G::sf(vm, l, mq + 5)]);
+            float2 w1 = make_float2(sF[G::sf(vp, l, m0 + 1)], sF[G::sf(vm, l, mq + 4)]);
+            float2 X2 = make_float2(sF[G::sf(vp, l, m0 + 2)], sF[G::sf(vm, l, mq + 3)]);
+            float2 X3 = make_float2(sF[G::sf(vp, l, m0 + 3)], sF[G::sf(vm, l, mq + 2)]);
+            float2 X4 = make_float2(sF[G::sf(vp, l, m0 + 4)], sF[G::sf(vm, l, mq + 1)]);
+            const float2 A10 = sub2_(w1, w0);
+            float2 A21 = sub2_(X2, w1), A32 = sub2_(X3, X2), A43 = sub2_(X4, X3);
+            float2 D0 = sub2_(A21, A10), D1 = sub2_(A32, A21), D2 = sub2_(A43, A32);
+            float2 DD0 = dd2_of(D0), DD1 = dd2_of(D1), DD2 = dd2_of(D2);
+            float gp[R + 1], gm[R + 1];
+#pragma unroll
+            for (int j = 0; j <= R; ++j) {
+                if (j == R && !last) break;
+                const int gmp = c0 + m0 + j;
+                // weno5z.cpp:80 on the inner '+' faces 3..n-3 (x only)
+                float2 DD2s = DD2;
+                if (zq && gmp >= 3 && gmp <= n - 3) DD2s.x = dd_of(A32.x);
+                const float2 fr =
+                    weno5_face_dq2<SCHEME>(X2, A21, A32, A43, D0, D2, DD0, DD1, DD2s);
+                gp[j] = fr.x;
+                gm[j] = fr.y;
+                if (j + 1 < K) {
+                    // '+' gains position m0+j+5, '-' position m0+K-1-j
+                    const float2 nw =
+                        make_float2(sF[G::sf(vp, l, m0 + j + 5)], sF[G::sf(vm, l, mq - j)]);
+                    X2 = X3;
+                    X3 = X4;
+                    X4 = nw;
+                    A21 = A32;
+                    A32 = A43;
+                    A43 = sub2_(X4, X3);
+                    D0 = D1;
+                    D1 = D2;
+                    D2 = sub2_(A43, A32);
+                    DD0 = DD1;
+                    DD1 = DD2;
+                    DD2 = dd2_of(D2);
+                }
+            }
+            // face k: '+' value gp[k], '-' value gm[K-1-k]
+#pragma unroll
+            for (int k = 0; k <= R; ++k) {
+                if (k == R && !last) break;
+                const float fmk = last ? gm[R - k] : gm[k < R ? R - 1 - k : 0];
+                Fh[k] = add_(gp[k], fmk);
+            }
         } else {
-            // FP64 runs of 4 faces step both windows together; the others step
-            // them one after the other (measured faster for FP32, and the joint
-            // form does not fit the 64-register budget of FP64 runs of 1 or 2)
-            constexpr bool joint = sizeof(B) == 8 && R == 4;
-            if constexpr (joint) {
-                // WENO5: each window carries the first differences a_ij, the second
-                // differences D and dd = 4 (13/12) D^2 of its current stencil, so each
-                // new face adds one value, one difference, one second difference
-                // and one square (weno5_face_dq).  The '+' stencil of face m is
-                // positions m..m+4, the '-' stencil m+5..m+1; both windows step
-                // together so that each face offers two independent chains.
-                const int vp = e, vm = 5 + e;
-                B p2 = sF[G::sf(vp, l, m0 + 2)], p3 = sF[G::sf(vp, l, m0 + 3)];
-                B p4 = sF[G::sf(vp, l, m0 + 4)];
-                B pa21, pa32, pa43, pD0, pD1, pD2;
-                {
-                    const B p0 = sF[G::sf(vp, l, m0)], p1 = sF[G::sf(vp, l, m0 + 1)];
-                    const B pa10 = sub_(p1, p0);
-                    pa21 = sub_(p2, p1);
-                    pa32 = sub_(p3, p2);
-                    pa43 = sub_(p4, p3);
-                    pD0 = sub_(pa21, pa10);
-                    pD1 = sub_(pa32, pa21);
-                    pD2 = sub_(pa43, pa32);
-                }
-                B pdd0 = dd_of(pD0), pdd1 = dd_of(pD1), pdd2 = dd_of(pD2);
-                B q0 = sF[G::sf(vm, l, m0 + 5)], q1 = sF[G::sf(vm, l, m0 + 4)];
-                B q2 = sF[G::sf(vm, l, m0 + 3)];
-                B qa10, qa21, qa32, qa43, qD0, qD1, qD2;
-                {
-                    const B q3 = sF[G::sf(vm, l, m0 + 2)], q4 = sF[G::sf(vm, l, m0 + 1)];
-                    qa10 = sub_(q1, q0);
-                    qa21 = sub_(q2, q1);
-                    qa32 = sub_(q3, q2);
-                    qa43 = sub_(q4, q3);
-                    qD0 = sub_(qa21, qa10);
-                    qD1 = sub_(qa32, qa21);
-                    qD2 = sub_(qa43, qa32);
-                }
-                B qdd0 = dd_of(qD0), qdd1 = dd_of(qD1), qdd2 = dd_of(qD2);
-                auto face = [&](int k) {
+            // WENO5: the window carries the first differences a_ij, the second
+            // differences D and dd = 4 (13/12) D^2 of the current stencil, so each
+            // new face adds one value, one difference, one second difference
+            // and one square (weno5_face_dq).
+            {  // '+' side: stencil f0..f4 = positions m..m+4
+                const int v = e;
+                B f0 = sF[G::sf(v, l, m0)], f1 = sF[G::sf(v, l, m0 + 1)];
+                B f2 = sF[G::sf(v, l, m0 + 2)], f3 = sF[G::sf(v, l, m0 + 3)];
+                B f4 = sF[G::sf(v, l, m0 + 4)];
+                B a10 = sub_(f1, f0), a21 = sub_(f2, f1), a32 = sub_(f3, f2), a43 = sub_(f4, f3);
+                B D0 = sub_(a21, a10), D1 = sub_(a32, a21), D2 = sub_(a43, a32);
+                B dd0 = dd_of(D0), dd1 = dd_of(D1), dd2 = dd_of(D2);
+#pragma unroll
+                for (int k = 0; k <= R; ++k) {
+                    if (k == R && !last) break;
                     const int gm = c0 + m0 + k;
                     // weno5z.cpp:80 on the inner '+' faces 3..n-3: beta2's first
                     // term reads f2 - 2 f3 + f3 = -a32
-                    const B dd2s = (zq && gm >= 3 && gm <= n - 3) ? dd_of(pa32) : pdd2;
-                    const B fp = weno5_face_dq<SCHEME, B>(p2, pa21, pa32, pa43, pD0, pD2, pdd0, pdd1, dd2s);
-                    const B fm = weno5_face_dq<SCHEME, B>(q2, qa21, qa32, qa43, qD0, qD2, qdd0, qdd1, qdd2);
-                    return add_(fp, fm);
-                };
-    #pragma unroll
-                for (int k = 0; k < R; ++k) {
-                    Fh[k] = face(k);
-                    // '+' gains position m0+k+5, '-' gains position m0+k+6
-                    p2 = p3;
-                    p3 = p4;
-                    p4 = sF[G::sf(vp, l, m0 + k + 5)];
-                    pa21 = pa32;
-                    pa32 = pa43;
-                    pa43 = sub_(p4, p3);
-                    pD0 = pD1;
-                    pD1 = pD2;
-                    pD2 = sub_(pa43, pa32);
-                    pdd0 = pdd1;
-                    pdd1 = pdd2;
-                    pdd2 = dd_of(pD2);
-                    const B qn = (m0 + k + 6 < NF) ? sF[G::sf(vm, l, m0 + k + 6)] : B(0);
-                    q2 = q1;
-                    q1 = q0;
-                    q0 = qn;
-                    qa43 = qa32;
-                    qa32 = qa21;
-                    qa21 = qa10;
-                    qa10 = sub_(q1, q0);
-                    qD2 = qD1;
-                    qD1 = qD0;
-                    qD0 = sub_(qa21, qa10);
-                    qdd2 = qdd1;
-                    qdd1 = qdd0;
-                    qdd0 = dd_of(qD0);
-                }
-                if (last) Fh[R] = face(R);
-            } else if constexpr (sizeof(B) == 4 && DIR == 0) {
-                // FP32 x sweep: faces in pairs on the packed f32x2 arithmetic.  The
-                // thread's K faces (R, and the next run's first on the last
-                // run) are taken '+' in ascending order beside '-' in
-                // descending order: the '+' stencil of face m0+j (positions
-                // m..m+4) and the '-' stencil of face m0+K-1-j (positions
-                // m'+5..m'+1) both step by dropping f0 and gaining a new f4,
-                // so one packed window (component x: '+', y: '-') carries
-                // both.  Component-wise the operations are those of the
-                // one-sided windows below, so every face is bitwise the same.
-                // (256^3 mixed step, x sweeps: WENO5-Z 1.895 -> 1.84 ms, WENO5-JS
-                // 1.81 -> 1.75 ms.  The y/z sweeps wait on their staging loads,
-                // not on FP32 issue: there the packed form measured the same
-                // (WENO5-Z) or 2-4 % slower (WENO5-JS), so they keep the
-                // one-sided form.)
-                const int K = R + (last ? 1 : 0);
-                const int mq = m0 + K - 1;  // the '-' side's first face
-                const int vp = e, vm = 5 + e;
-                float2 w0 = make_float2(sF[G::sf(vp, l, m0)], sF[G::sf(vm, l, mq + 5)]);
-                float2 w1 = make_float2(sF[G::sf(vp, l, m0 + 1)], sF[G::sf(vm, l, mq + 4)]);
-                float2 X2 = make_float2(sF[G::sf(vp, l, m0 + 2)], sF[G::sf(vm, l, mq + 3)]);
-                float2 X3 = make_float2(sF[G::sf(vp, l, m0 + 3)], sF[G::sf(vm, l, mq + 2)]);
-                float2 X4 = make_float2(sF[G::sf(vp, l, m0 + 4)], sF[G::sf(vm, l, mq + 1)]);
-                const float2 A10 = sub2_(w1, w0);
-                float2 A21 = sub2_(X2, w1), A32 = sub2_(X3, X2), A43 = sub2_(X4, X3);
-                float2 D0 = sub2_(A21, A10), D1 = sub2_(A32, A21), D2 = sub2_(A43, A32);
-                float2 DD0 = dd2_of(D0), DD1 = dd2_of(D1), DD2 = dd2_of(D2);
-                float gp[R + 1], gm[R + 1];
-    #pragma unroll
-                for (int j = 0; j <= R; ++j) {
-                    if (j == R && !last) break;
-                    const int gmp = c0 + m0 + j;
-                    // weno5z.cpp:80 on the inner '+' faces 3..n-3 (x only)
-                    float2 DD2s = DD2;
-                    if (zq && gmp >= 3 && gmp <= n - 3) DD2s.x = dd_of(A32.x);
-                    const float2 fr =
-                        weno5_face_dq2<SCHEME>(X2, A21, A32, A43, D0, D2, DD0, DD1, DD2s);
-                    gp[j] = fr.x;
-                    gm[j] = fr.y;
-                    if (j + 1 < K) {
-                        // '+' gains position m0+j+5, '-' position m0+K-1-j
-                        const float2 nw =
-                            make_float2(sF[G::sf(vp, l, m0 + j + 5)], sF[G::sf(vm, l, mq - j)]);
-                        X2 = X3;
-                        X3 = X4;
-                        X4 = nw;
-                        A21 = A32;
-                        A32 = A43;
-                        A43 = sub2_(X4, X3);
+                    const B dd2s = (zq && gm >= 3 && gm <= n - 3) ? dd_of(a32) : dd2;
+                    Fh[k] = weno5_face_dq<SCHEME>(f2, a21, a32, a43, D0, D2, dd0, dd1, dd2s);
+                    if (k < R) {
+                        f2 = f3;
+                        f3 = f4;
+                        f4 = sF[G::sf(v, l, m0 + k + 5)];
+                        a21 = a32;
+                        a32 = a43;
+                        a43 = sub_(f4, f3);
                         D0 = D1;
                         D1 = D2;
-                        D2 = sub2_(A43, A32);
-                        DD0 = DD1;
-                        DD1 = DD2;
-                        DD2 = dd2_of(D2);
+                        D2 = sub_(a43, a32);
+                        dd0 = dd1;
+                        dd1 = dd2;
+                        dd2 = dd_of(D2);
                     }
                 }
-                // face k: '+' value gp[k], '-' value gm[K-1-k]
-    #pragma unroll
+            }
+            {  // '-' side: stencil f0..f4 = positions m+5..m+1
+                const int v = 5 + e;
+                B f0 = sF[G::sf(v, l, m0 + 5)], f1 = sF[G::sf(v, l, m0 + 4)];
+                B f2 = sF[G::sf(v, l, m0 + 3)], f3 = sF[G::sf(v, l, m0 + 2)];
+                B f4 = sF[G::sf(v, l, m0 + 1)];
+                B a10 = sub_(f1, f0), a21 = sub_(f2, f1), a32 = sub_(f3, f2), a43 = sub_(f4, f3);
+                B D0 = sub_(a21, a10), D1 = sub_(a32, a21), D2 = sub_(a43, a32);
+                B dd0 = dd_of(D0), dd1 = dd_of(D1), dd2 = dd_of(D2);
+#pragma unroll
                 for (int k = 0; k <= R; ++k) {
                     if (k == R && !last) break;
-                    const float fmk = last ? gm[R - k] : gm[k < R ? R - 1 - k : 0];
-                    Fh[k] = add_(gp[k], fmk);
-                }
-            } else {
-                // WENO5: the window carries the first differences a_ij, the second
-                // differences D and dd = 4 (13/12) D^2 of the current stencil, so each
-                // new face adds one value, one difference, one second difference
-                // and one square (weno5_face_dq).
-                {  // '+' side: stencil f0..f4 = positions m..m+4
-                    const int v = e;
-                    B f0 = sF[G::sf(v, l, m0)], f1 = sF[G::sf(v, l, m0 + 1)];
-                    B f2 = sF[G::sf(v, l, m0 + 2)], f3 = sF[G::sf(v, l, m0 + 3)];
-                    B f4 = sF[G::sf(v, l, m0 + 4)];
-                    B a10 = sub_(f1, f0), a21 = sub_(f2, f1), a32 = sub_(f3, f2), a43 = sub_(f4, f3);
-                    B D0 = sub_(a21, a10), D1 = sub_(a32, a21), D2 = sub_(a43, a32);
-                    B dd0 = dd_of(D0), dd1 = dd_of(D1), dd2 = dd_of(D2);
-    #pragma unroll
-                    for (int k = 0; k <= R; ++k) {
-                        if (k == R && !last) break;
-                        const int gm = c0 + m0 + k;
-                        // weno5z.cpp:80 on the inner '+' faces 3..n-3: beta2's first
-                        // term reads f2 - 2 f3 + f3 = -a32
-                        const B dd2s = (zq && gm >= 3 && gm <= n - 3) ? dd_of(a32) : dd2;
-                        Fh[k] = weno5_face_dq<SCHEME, B>(f2, a21, a32, a43, D0, D2, dd0, dd1, dd2s);
-                        if (k < R) {
-                            f2 = f3;
-                            f3 = f4;
-                            f4 = sF[G::sf(v, l, m0 + k + 5)];
-                            a21 = a32;
-                            a32 = a43;
-                            a43 = sub_(f4, f3);
-                            D0 = D1;
-                            D1 = D2;
-                            D2 = sub_(a43, a32);
-                            dd0 = dd1;
-                            dd1 = dd2;
-                            dd2 = dd_of(D2);
-                        }
-                    }
-                }
-                {  // '-' side: stencil f0..f4 = positions m+5..m+1
-                    const int v = 5 + e;
-                    B f0 = sF[G::sf(v, l, m0 + 5)], f1 = sF[G::sf(v, l, m0 + 4)];
-                    B f2 = sF[G::sf(v, l, m0 + 3)], f3 = sF[G::sf(v, l, m0 + 2)];
-                    B f4 = sF[G::sf(v, l, m0 + 1)];
-                    B a10 = sub_(f1, f0), a21 = sub_(f2, f1), a32 = sub_(f3, f2), a43 = sub_(f4, f3);
-                    B D0 = sub_(a21, a10), D1 = sub_(a32, a21), D2 = sub_(a43, a32);
-                    B dd0 = dd_of(D0), dd1 = dd_of(D1), dd2 = dd_of(D2);
-    #pragma unroll
-                    for (int k = 0; k <= R; ++k) {
-                        if (k == R && !last) break;
-                        Fh[k] = add_(Fh[k], weno5_face_dq<SCHEME, B>(f2, a21, a32, a43, D0, D2, dd0,
-                                                                     dd1, dd2));
-                        if (k < R) {
-                            const B fn = (m0 + k + 6 < NF) ? sF[G::sf(v, l, m0 + k + 6)] : B(0);
-                            f2 = f1;
-                            f1 = f0;
-                            f0 = fn;
-                            a43 = a32;
-                            a32 = a21;
-                            a21 = a10;
-                            a10 = sub_(f1, f0);
-                            D2 = D1;
-                            D1 = D0;
-                            D0 = sub_(a21, a10);
-                            dd2 = dd1;
-                            dd1 = dd0;
-                            dd0 = dd_of(D0);
-                        }
+                    Fh[k] = add_(Fh[k], weno5_face_dq<SCHEME>(f2, a21, a32, a43, D0, D2, dd0,
+                                                                 dd1, dd2));
+                    if (k < R) {
+                        const B fn = (m0 + k + 6 < NF) ? sF[G::sf(v, l, m0 + k + 6)] : B(0);
+                        f2 = f1;
+                        f1 = f0;
+                        f0 = fn;
+                        a43 = a32;
+                        a32 = a21;
+                        a21 = a10;
+                        a10 = sub_(f1, f0);
+                        D2 = D1;
+                        D1 = D0;
+                        D0 = sub_(a21, a10);
+                        dd2 = dd1;
+                        dd1 = dd0;
+                        dd0 = dd_of(D0);
                     }
                 }
             }

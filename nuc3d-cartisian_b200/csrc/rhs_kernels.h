@@ -117,8 +117,9 @@ cudaError_t launch_residual(const BoxDev *boxes, int nboxes, cudaStream_t st);
 cudaError_t launch_clear_eig(const BoxDev *boxes, int nboxes, cudaStream_t st);
 // variant v of the sweep kernel: tiles of kInvTileCells[v] cells along the
 // sweep, runs of kInvRunLen[v] faces per thread (picked per scheme and
-// direction by the engine's autotuner); variants 0-2 use 32-cell tiles, 3-4
-// 64-cell tiles (their work items differ: kInvTileClass)
+// direction by the engine's autotuner; the pairs of marched() read the variant
+// as march_cells()); variants 0-2 use 32-cell tiles, 3-4 64-cell tiles (their
+// work items differ: inv_tile_class)
 constexpr int kInvVariants = 5;
 constexpr int kInvTileCells[kInvVariants] = {32, 32, 32, 64, 64};
 constexpr int kInvRunLen[kInvVariants] = {1, 2, 4, 2, 4};
