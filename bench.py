@@ -77,11 +77,11 @@ FLOPS_INV_LAUNCH = FLOPS_INV_Z + FLOPS_PRIM / 3
 STATE_BYTES_PER_CELL_UPDATE = 320  # compulsory FP64 state traffic of 3 RK stages
 # DRAM bytes (read + write) per launch of the FP64 WENO5-Z sweep at 256^3,
 # mean of x, y, z: the ncu capture at 128^3 in
-# profiles/k_inviscid_weno5z_fp64_128.md (212.0, 269.4, 281.8 MB; the x sweep
+# profiles/sweeps_weno5z_fp64_128.md (226.8, 274.1, 272.9 MB; the x sweep
 # reads the state only and writes the primitives as well as its RHS) scaled
 # by the cell count (x8); the traffic of a sweep is proportional to the cells
 # it covers (whole lines, no halo growth with size along the other axes).
-INV_TRAFFIC_BYTES = 8 * (212.03072e6 + 269.391872e6 + 281.837568e6) / 3
+INV_TRAFFIC_BYTES = 8 * (226.784768e6 + 274.140928e6 + 272.945664e6) / 3
 INV_TRAFFIC_NOTE = "ncu dram__bytes_read+write of the 128^3 capture x8 (cells), mean of x/y/z"
 
 
@@ -323,7 +323,7 @@ def run_b200(args, rank, world, local_rank):
     achieved = FLOPS_INV_LAUNCH * cells / (inv_avg_ms * 1e-3) / 1e12
     roofline = {
         "bound": "fp64",
-        "kernel": "k_inviscid<WENO5-Z, FP64> (directional sweep, x/y/z; x also recovers the primitives)",
+        "kernel": "k_xsweep (x, with con2prim) and k_march (y, z), WENO5-Z, FP64: mean of the three launches",
         "achieved": achieved,
         "peak": peak64,
         "unit": "TFLOP/s",
