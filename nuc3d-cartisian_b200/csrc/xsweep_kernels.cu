@@ -250,6 +250,9 @@ __global__ void __launch_bounds__(kThreads, SCHEME == SCHEME_W7 ? 3 : 4)
             }
             const double left = __shfl_up_sync(0xffffffffu, S[RUN - 1], 1);
             if (r > 0) S0 = left;
+            // a line's lanes share a warp: its r = 0 has read the tile before's face
+            // (a shuffle alone orders no memory) before r = NR-1 replaces it
+            __syncwarp();
             if (r == NR - 1) sC[e * TL + l] = S[RUN - 1];
 #pragma unroll
             for (int k = RUN - 1; k >= 0; --k) {
