@@ -659,13 +659,15 @@ cudaError_t op_lines(int sch, int upwind, int nx, long long lines, const double 
     const int ms = crweno_segment_rows(sch, nx, true), P = crweno_lanes(sch, nx, true);
     const int N = line_unknowns(sch, nx, true);
     const size_t per = sizeof(double) * (size_t)(nx + 2 * scheme_halo(sch) + 3 * ms * 32);
-    const size_t fit = (size_t)200 * 1024 / per;  // nx = 4096: 131 KB, one warp
+    constexpr int kMaxSmem = 200 * 1024;
+    const size_t fit = (size_t)kMaxSmem / per;  // nx = 4096: 131 KB, one warp
     const int warps = (int)(fit < 8 ? fit : 8);
     const auto k = sch == SCHEME_HC    ? k_op_lines<SCHEME_HC>
                    : sch == SCHEME_H77 ? k_op_lines<SCHEME_H77>
                                        : k_op_lines<SCHEME_CR>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(per * warps));
+    // (the attribute belongs to the process, so every call sets the same value:
+    // with its own need a call would lower the limit under another thread's launch)
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e != cudaSuccess) return e;
     k<<<(unsigned)((lines + warps - 1) / warps), 32 * warps, per * warps, st>>>(
         upwind > 0 ? 0 : 1, nx, lines, ms, N, P, in, hl, hr, out);

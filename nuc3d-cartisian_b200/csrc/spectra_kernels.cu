@@ -272,14 +272,13 @@ cudaError_t launch_spectra(const BoxDev &b, const SpectraPlan &plan, void *scrat
     if (r != CUFFT_SUCCESS) return cudaSuccess;
     // warps per block: as many shell tables as fit 200 KB, at most 8 (a box
     // of 2^31 cells has kmax <= 645)
+    constexpr int kMaxSmem = 200 * 1024;
     const size_t table = sizeof(double) * kSpectra * (size_t)(kmax + 1);
-    const int warps = (int)(200 * 1024 / table < 8 ? 200 * 1024 / table : 8);
+    const int warps = (int)(kMaxSmem / table < 8 ? kMaxSmem / table : 8);
     const size_t smem = table * warps;
-    if (smem > 48 * 1024) {
-        e = cudaFuncSetAttribute(k_spec_bin, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    // (the same limit from every call: it is shared with the other host threads)
+    e = cudaFuncSetAttribute(k_spec_bin, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    if (e != cudaSuccess) return e;
     k_spec_bin<<<kSpecBlocks, 32 * warps, smem, st>>>(reinterpret_cast<const double2 *>(F), p.n[0],
                                                     p.n[1], p.n[2], kmax, partials);
     const int n = kSpectra * kmax;
