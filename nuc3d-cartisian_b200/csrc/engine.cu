@@ -222,6 +222,16 @@ bool step_fork_enabled() {
     return !(env && env[0] == '0');
 }
 
+// the pencil depth that NUC3D_PENCIL_DEPTH pins (index into kPencilDepths; the
+// default depth for a value that is none), -1 without it
+int pinned_pencil() {
+    const char *env = std::getenv("NUC3D_PENCIL_DEPTH");
+    if (!env) return -1;
+    for (int v = 0; v < kPencils; ++v)
+        if (kPencilDepths[v] == std::atoi(env)) return v;
+    return 0;
+}
+
 // the flags pointers of up to kMax boxes, passed by value to k_export_flags
 struct FlagPtrs {
     static constexpr int kMax = 32;
@@ -237,7 +247,7 @@ __global__ void k_export_flags(FlagPtrs f, unsigned *out) {
 
 Engine::Engine(int precision, cudaStream_t stream) : precision_(precision), stream_(stream) {
     cudaGetDevice(&device_);
-    std::fill(pencil_of_class, pencil_of_class + kPencilClasses, (signed char)-1);
+    for (auto &p : pencil_of_class) std::fill(p, p + kPencilClasses, (signed char)-1);
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -468,14 +478,20 @@ int Engine::rebuild() {
     ECK(cudaStreamSynchronize(stream_));
     const bool mixed = precision_ == NUC3D_MIXED;
     std::vector<BoxDev> table(boxes_.size());
-    std::vector<WorkItem> prim, st25[kVisClasses], inv[kSchemes][3][kInvTileClasses],
+    std::vector<WorkItem> prim, st25[kVisClasses][kPencils], inv[kSchemes][3][kInvTileClasses],
         march[kSchemes][3], thomas[3], cr[kLineSchemes][3];
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d) march_nmax_[s][d] = 0;
     const int crtl = crweno_tile_lines();
     for (int c = 0; c < kLineSchemes; ++c)
         for (int d = 0; d < 3; ++d) cr_nmax_[c][d] = cr_ms_[c][d] = 0;
-    for (int c = 0; c < kVisClasses; ++c) nzmax_[c] = 0;
+    // (blocks of the 2.5-D kernels at 16 planes)
+    long long blocks16 = 0;
+    for (const EngineBox &b : boxes_)
+        if (b.live && b.dev.active)
+            blocks16 += (long long)ceil_div(b.dev.p.n[0], kT25X) * ceil_div(b.dev.p.n[1], kT25Y) *
+                        ceil_div(b.dev.p.n[2], 16);
+    short_pencils_ = blocks16 <= kPencilShortBlocks || pinned_pencil() >= kLongPencils;
     any_visc_ = false;
     nactive_ = 0;
     active_cells_ = 0;
@@ -494,9 +510,11 @@ int Engine::rebuild() {
             prim.push_back({id, (int)c, (int)std::min<long long>(kPrimChunk, p.N - c * kPrimChunk), 0});
         boxes_[i].prim_n = (int)prim.size() - boxes_[i].prim_off;
         const int vc = vis_class(p);
-        nzmax_[vc] = std::max(nzmax_[vc], p.n[2]);
-        for (int y = 0; y < ceil_div(p.n[1], kT25Y); ++y)
-            for (int x = 0; x < ceil_div(p.n[0], kT25X); ++x) st25[vc].push_back({id, x, y, 0});
+        for (int v = 0; v < (short_pencils_ ? kPencils : kLongPencils); ++v)
+            for (int z = 0; z < ceil_div(p.n[2], kPencilDepths[v]); ++z)
+                for (int y = 0; y < ceil_div(p.n[1], kT25Y); ++y)
+                    for (int x = 0; x < ceil_div(p.n[0], kT25X); ++x)
+                        st25[vc][v].push_back({id, x, y, z});
         for (int d = 0; d < 3; ++d) {
             int s = p.scheme[d];
             if (line_slot(s) >= 0) {
@@ -556,7 +574,8 @@ int Engine::rebuild() {
         all.insert(all.end(), v.begin(), v.end());
     };
     append(prim, r_prim_);
-    for (int c = 0; c < kVisClasses; ++c) append(st25[c], r_25d_[c]);
+    for (int c = 0; c < kVisClasses; ++c)
+        for (int v = 0; v < kPencils; ++v) append(st25[c][v], r_25d_[c][v]);
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d)
             for (int tc = 0; tc < kInvTileClasses; ++tc) append(inv[s][d][tc], r_inv_[s][d][tc]);
@@ -593,7 +612,7 @@ int Engine::rebuild() {
     ECK(prepare_stencil_kernels(mixed));
     int per_stage = 0;
     for (int c = 0; c < kVisClasses; ++c)
-        per_stage += (any_visc_ && r_25d_[c].n > 0) + (r_25d_[c].n > 0);
+        per_stage += (any_visc_ && r_25d_[c][0].n > 0) + (r_25d_[c][0].n > 0);
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d) per_stage += has_sweep(s, d);
     for (int c = 0; c < kLineSchemes; ++c)
@@ -742,9 +761,9 @@ cudaError_t Engine::launch_sweep(int s, int d, int v, int in, int prim_mode, cud
 template <typename B>
 cudaError_t Engine::launch_visc_classes(int v, cudaStream_t st) {
     for (int c = 0; c < kVisClasses; ++c) {
-        const Range &rg = r_25d_[c];
-        cudaError_t e = launch_visc_flux<B>(d_boxes_, d_items_ + rg.off, rg.n, nzmax_[c],
-                                            kPencilDepths[v], kVisReach[c], st);
+        const Range &rg = r_25d_[c][v];
+        cudaError_t e = launch_visc_flux<B>(d_boxes_, d_items_ + rg.off, rg.n, kPencilDepths[v],
+                                            kVisReach[c], st);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -753,9 +772,9 @@ cudaError_t Engine::launch_visc_classes(int v, cudaStream_t st) {
 template <typename B>
 cudaError_t Engine::launch_update_classes(int v, StageArgs sa, cudaStream_t st) {
     for (int c = 0; c < kVisClasses; ++c) {
-        const Range &rg = r_25d_[c];
-        cudaError_t e = launch_update<B>(d_boxes_, d_items_ + rg.off, rg.n, nzmax_[c],
-                                         kPencilDepths[v], sa, any_visc_, kVisReach[c], st);
+        const Range &rg = r_25d_[c][v];
+        cudaError_t e = launch_update<B>(d_boxes_, d_items_ + rg.off, rg.n, kPencilDepths[v], sa,
+                                         any_visc_, kVisReach[c], st);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -791,24 +810,18 @@ int Engine::enqueue_step(cudaStream_t s) {
 // update is timed as a first stage, which writes only the u1 slot that the
 // next step's first stage overwrites (and no residual), so timing on the
 // live state changes nothing.
-long long Engine::pencil_blocks(int v) const {
-    long long b = 0;
-    for (int c = 0; c < kVisClasses; ++c)
-        b += (long long)r_25d_[c].n * ceil_div(nzmax_[c], kPencilDepths[v]);
-    return b;
-}
-
 int Engine::autotune() {
     bool need_sweep = false;
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d)
             need_sweep = need_sweep || (has_sweep(s, d) && inv_variant[s][d] < 0);
-    const bool stencils = r_25d_[0].n > 0 || r_25d_[1].n > 0;
+    const bool stencils = r_25d_[0][0].n > 0 || r_25d_[1][0].n > 0;
     int cls = 0;  // size class: floor(log4(active cells))
     while (cls + 1 < kPencilClasses && (active_cells_ >> (2 * (cls + 1))) > 0) ++cls;
-    const bool need_pencil = stencils && pencil_of_class[cls] < 0;
-    if (stencils && !need_pencil && pencil_variant != pencil_of_class[cls]) {
-        pencil_variant = pencil_of_class[cls];
+    signed char &kept_pencil = pencil_of_class[short_pencils_][cls];
+    const bool need_pencil = stencils && kept_pencil < 0;
+    if (stencils && !need_pencil && pencil_variant != kept_pencil) {
+        pencil_variant = kept_pencil;
         invalidate_graph();
     }
     if (!need_sweep && !need_pencil) return NUC3D_OK;
@@ -833,12 +846,11 @@ int Engine::autotune() {
     }
     bool tune_pencil = need_pencil;
     if (need_pencil) {
-        if (const char *pin = std::getenv("NUC3D_PENCIL_DEPTH")) {
-            const int want = std::atoi(pin);
-            pencil_variant = 0;
-            for (int v = 0; v < kPencils; ++v)
-                if (kPencilDepths[v] == want) pencil_variant = v;
-            pencil_of_class[cls] = (signed char)pencil_variant;
+        const int pin = pinned_pencil();
+        if (pin >= 0) {
+            // (a short depth has work lists if it was pinned at the rebuild)
+            pencil_variant = pin >= kLongPencils && !short_pencils_ ? 0 : pin;
+            kept_pencil = (signed char)pencil_variant;
             tune_pencil = false;
         }
     }
@@ -897,7 +909,7 @@ int Engine::autotune() {
             // the best so far
             const int longer = v == 3 ? 1 : v - 1;
             if ((v == 2 && best == 1) ||
-                (v > 2 && (pencil_blocks(1) > kPencilShortBlocks || best != longer))) {
+                (v >= kLongPencils && (!short_pencils_ || best != longer))) {
                 pencil_tune_ms[v] = 0.0;
                 continue;
             }
@@ -915,7 +927,7 @@ int Engine::autotune() {
             if (ms < pencil_tune_ms[best]) best = v;
         }
         pencil_variant = best;
-        pencil_of_class[cls] = (signed char)best;
+        kept_pencil = (signed char)best;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

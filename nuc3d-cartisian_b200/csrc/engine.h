@@ -90,12 +90,13 @@ public:
     // autotuned pencil depth of the 2.5-D stencil kernels: index into
     // kPencilDepths (-1: not tuned yet), the measured milliseconds of one
     // viscous-flux + update pass per depth of the last tuning, and the depth
-    // found for each power of four of active cells (a batch that grows or
-    // shrinks into a size class it has been in takes that class's depth)
+    // found for each power of four of active cells with and without the short
+    // depths (a batch that grows or shrinks into a size class it has been in
+    // takes that class's depth)
     int pencil_variant = -1;
     double pencil_tune_ms[kPencils] = {};
     static constexpr int kPencilClasses = 20;
-    signed char pencil_of_class[kPencilClasses];
+    signed char pencil_of_class[2][kPencilClasses];
 
     static long long box_bytes(const nuc3d_box_desc &d);
     static int validate(const nuc3d_box_desc &d, std::string *why);
@@ -169,12 +170,11 @@ private:
     // variant v of the directional sweep of scheme s on this batch's boxes
     template <typename B>
     cudaError_t launch_sweep(int s, int d, int v, int in, int prim_mode, cudaStream_t st);
-    // 2.5-D stencil tiles per stencil class (kVisReach), and the most planes
-    // among its boxes
-    Range r_25d_[kVisClasses];
-    int nzmax_[kVisClasses] = {};
+    // 2.5-D stencil tiles per [stencil class (kVisReach)][pencil depth of
+    // kPencilDepths]; the short depths' lists only where short_pencils_
+    Range r_25d_[kVisClasses][kPencils];
+    bool short_pencils_ = false;
     long long active_cells_ = 0;
-    long long pencil_blocks(int v) const;  // blocks of a 2.5-D launch at depth v
     // blocks up to which the short pencils are worth timing: two waves of 148
     // SMs x 2 blocks at depth 16
     static constexpr long long kPencilShortBlocks = 600;

@@ -103,7 +103,11 @@ constexpr int kT25X = 32, kT25Y = 8;  // 2.5-D tile of the stencil kernels (x, y
 // ones are for boxes whose tiles leave the SMs idle: a plane costs a block
 // about 1.7 us of latency, so at 16 planes a 32^3 box (8 blocks) spent 28 us
 // in the viscous-flux kernel and 35 us in the update, at 4 planes 13 and 15.
-constexpr int kPencils = 6;
+// The chunk stands in the work item, so a box makes only its own blocks whatever
+// else is in the batch and any number of planes fits; as a grid dimension (at
+// most 65535, of the tallest box) it also cost the update registers: mixed
+// 120^3, 79.4 against 77.1 us.
+constexpr int kPencils = 6, kLongPencils = 3;  // the first kLongPencils suit any box
 constexpr int kPencilDepths[kPencils] = {32, 16, 64, 8, 4, 2};
 constexpr int kPrimChunk = 4096;                  // cells per k_prim work item
 
@@ -185,14 +189,14 @@ cudaError_t prepare_stencil_kernels(bool mixed);
 // scheme as coefficients, BoxParams::vcoef).
 constexpr int kVisClasses = 2;
 constexpr int kVisReach[kVisClasses] = {3, 4};
-// nzmax: the most planes among the launch's boxes; depth: planes per block;
+// depth: planes per work item along z (the items' z chunks are of that size);
 // reach: the stencil class's reach (3 or 4)
 template <typename B>
-cudaError_t launch_visc_flux(const BoxDev *boxes, const WorkItem *items, int nitems, int nzmax,
-                             int depth, int reach, cudaStream_t st);
+cudaError_t launch_visc_flux(const BoxDev *boxes, const WorkItem *items, int nitems, int depth,
+                             int reach, cudaStream_t st);
 template <typename B>
-cudaError_t launch_update(const BoxDev *boxes, const WorkItem *items, int nitems, int nzmax,
-                          int depth, StageArgs sa, bool any_viscous, int reach, cudaStream_t st);
+cudaError_t launch_update(const BoxDev *boxes, const WorkItem *items, int nitems, int depth,
+                          StageArgs sa, bool any_viscous, int reach, cudaStream_t st);
 
 // CRWENO5 / hccs sweeps (crweno_kernels.cu), batched: one work item per tile of
 // crweno_tile_lines() lines of one box.  nmax is the longest line among the

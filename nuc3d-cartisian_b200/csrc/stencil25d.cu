@@ -109,7 +109,7 @@ __device__ __forceinline__ T cd_any(T m4, T m3, T m2, T m1, T p1, T p2, T p3, T 
 // u, v, w, T by the differential schemes (FP64 differences), stresses and
 // heat flux in the bulk type, written as tau_xx, tau_xy, tau_xz, tau_yy,
 // tau_yz, tau_zz, E_x, E_y, E_z.
-// Work item: (box, x tile, y tile); blockIdx.y: the z chunk of `depth` planes.
+// Work item: (box, x tile, y tile, z chunk of `depth` planes).
 template <typename B, int R>
 __global__ void __launch_bounds__(TX *TY, 2) k_visc_flux25(const BoxDev *__restrict__ boxes, const WorkItem *__restrict__ items, int depth) {
     // dynamic shared memory (visc_smem_bytes): the two plane tiles with their
@@ -140,8 +140,7 @@ __global__ void __launch_bounds__(TX *TY, 2) k_visc_flux25(const BoxDev *__restr
     B *const vbase = fieldV<B>(bd, 0);
     const int nx = bp.n[0], ny = bp.n[1], nz = bp.n[2];
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-    const int i0 = it.a * TX, j0 = it.b * TY, k0 = blockIdx.y * depth;
-    if (k0 >= nz) return;  // the launch's longest box sets the grid
+    const int i0 = it.a * TX, j0 = it.b * TY, k0 = it.c * depth;
     const int i = i0 + tx, j = j0 + ty;
     const bool active = i < nx && j < ny;
     const long long sz = bp.stride[2];
@@ -316,7 +315,7 @@ __global__ void __launch_bounds__(TX *TY, 2) k_visc_flux25(const BoxDev *__restr
 // TVD-RK3 stage (TVD-RK3.cpp:76-196, dQ/dt = -RHS) in FP64; on the last stage
 // also the residual sum of PDEData3d::setRES (PDEData3d.cpp:178-213).  Every
 // new state value passes a finite check.  stage = -1 writes the total RHS.
-// Work item: (box, x tile, y tile); blockIdx.y: the z chunk.  ANYVIS: some box of the batch
+// Work item: (box, x tile, y tile, z chunk of `depth` planes).  ANYVIS: some box of the batch
 // is viscous (sizes the shared tiles); per box the viscous part runs only for
 // Navier-Stokes boxes.
 template <typename B, bool ANYVIS, int R>
@@ -371,8 +370,7 @@ __global__ void __launch_bounds__(TX *TY, 2)
     const StepScalars *sc = bd.sc;
     const int nx = bp.n[0], ny = bp.n[1], nz = bp.n[2];
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-    const int i0 = it.a * TX, j0 = it.b * TY, k0 = blockIdx.y * depth;
-    if (k0 >= nz) return;  // the launch's longest box sets the grid
+    const int i0 = it.a * TX, j0 = it.b * TY, k0 = it.c * depth;
     const int i = i0 + tx, j = j0 + ty;
     const bool active = i < nx && j < ny;
     const long long sz = bp.stride[2];
@@ -557,38 +555,38 @@ cudaError_t prepare_stencil_kernels(bool mixed) {
 }
 
 template <typename B>
-cudaError_t launch_visc_flux(const BoxDev *boxes, const WorkItem *items, int nitems, int nzmax,
-                             int depth, int reach, cudaStream_t st) {
+cudaError_t launch_visc_flux(const BoxDev *boxes, const WorkItem *items, int nitems, int depth,
+                             int reach, cudaStream_t st) {
     if (nitems <= 0) return cudaSuccess;
-    const dim3 grid(nitems, (nzmax + depth - 1) / depth), block(TX, TY);
+    const dim3 block(TX, TY);
     if (reach == 3)
-        k_visc_flux25<B, 3><<<grid, block, visc_smem_bytes(3), st>>>(boxes, items, depth);
+        k_visc_flux25<B, 3><<<nitems, block, visc_smem_bytes(3), st>>>(boxes, items, depth);
     else
-        k_visc_flux25<B, 4><<<grid, block, visc_smem_bytes(4), st>>>(boxes, items, depth);
+        k_visc_flux25<B, 4><<<nitems, block, visc_smem_bytes(4), st>>>(boxes, items, depth);
     return cudaGetLastError();
 }
 
 template <typename B>
-cudaError_t launch_update(const BoxDev *boxes, const WorkItem *items, int nitems, int nzmax,
-                          int depth, StageArgs sa, bool any_viscous, int reach, cudaStream_t st) {
+cudaError_t launch_update(const BoxDev *boxes, const WorkItem *items, int nitems, int depth,
+                          StageArgs sa, bool any_viscous, int reach, cudaStream_t st) {
     if (nitems <= 0) return cudaSuccess;
-    const dim3 grid(nitems, (nzmax + depth - 1) / depth), block(TX, TY);
+    const dim3 block(TX, TY);
     if (!any_viscous)
-        k_update25<B, false, 3><<<grid, block, 0, st>>>(boxes, items, depth, sa);
+        k_update25<B, false, 3><<<nitems, block, 0, st>>>(boxes, items, depth, sa);
     else if (reach == 3)
-        k_update25<B, true, 3><<<grid, block, 0, st>>>(boxes, items, depth, sa);
+        k_update25<B, true, 3><<<nitems, block, 0, st>>>(boxes, items, depth, sa);
     else
-        k_update25<B, true, 4><<<grid, block, update_smem_bytes<B>(), st>>>(boxes, items, depth, sa);
+        k_update25<B, true, 4><<<nitems, block, update_smem_bytes<B>(), st>>>(boxes, items, depth, sa);
     return cudaGetLastError();
 }
 
-template cudaError_t launch_visc_flux<double>(const BoxDev *, const WorkItem *, int, int, int, int,
+template cudaError_t launch_visc_flux<double>(const BoxDev *, const WorkItem *, int, int, int,
                                               cudaStream_t);
-template cudaError_t launch_visc_flux<float>(const BoxDev *, const WorkItem *, int, int, int, int,
+template cudaError_t launch_visc_flux<float>(const BoxDev *, const WorkItem *, int, int, int,
                                              cudaStream_t);
-template cudaError_t launch_update<double>(const BoxDev *, const WorkItem *, int, int, int,
+template cudaError_t launch_update<double>(const BoxDev *, const WorkItem *, int, int,
                                            StageArgs, bool, int, cudaStream_t);
-template cudaError_t launch_update<float>(const BoxDev *, const WorkItem *, int, int, int,
+template cudaError_t launch_update<float>(const BoxDev *, const WorkItem *, int, int,
                                           StageArgs, bool, int, cudaStream_t);
 
 }  // namespace nuc3d
