@@ -5,6 +5,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -222,7 +223,21 @@ bool step_fork_enabled() {
     return !(env && env[0] == '0');
 }
 
-// the pencil depth that NUC3D_PENCIL_DEPTH pins (index into kPencilDepths; the
+// the sweep variant that NUC3D_SWEEP_RUN=1|2|4 pins (32-cell tiles; with
+// NUC3D_SWEEP_TILE=64, runs of 2 or 4 on 64-cell tiles, not in mixed precision;
+// for marched pairs the five name the chunk lengths), -1 without it
+int pinned_sweep(bool mixed) {
+    const char *env = std::getenv("NUC3D_SWEEP_RUN");
+    if (!env) return -1;
+    const int run = std::atoi(env);
+    const char *tile = std::getenv("NUC3D_SWEEP_TILE");
+    const int tc = tile && std::atoi(tile) == 64 && run != 1 && !mixed ? 64 : 32;
+    int v = 2;
+    for (int k = 0; k < kInvVariants; ++k)
+        if (kInvRunLen[k] == run && kInvTileCells[k] == tc) v = k;
+    return v;
+}
+// the pencil depth that NUC3D_PENCIL_DEPTH=2|4|8|16|32|64 pins (index into kPencilDepths; the
 // default depth for a value that is none), -1 without it
 int pinned_pencil() {
     const char *env = std::getenv("NUC3D_PENCIL_DEPTH");
@@ -479,9 +494,7 @@ int Engine::rebuild() {
     const bool mixed = precision_ == NUC3D_MIXED;
     std::vector<BoxDev> table(boxes_.size());
     std::vector<WorkItem> prim, st25[kVisClasses][kPencils], inv[kSchemes][3][kInvTileClasses],
-        march[kSchemes][3], thomas[3], cr[kLineSchemes][3];
-    for (int s = 0; s < kSchemes; ++s)
-        for (int d = 0; d < 3; ++d) march_nmax_[s][d] = 0;
+        thomas[3], cr[kLineSchemes][3];
     const int crtl = crweno_tile_lines();
     for (int c = 0; c < kLineSchemes; ++c)
         for (int d = 0; d < 3; ++d) cr_nmax_[c][d] = cr_ms_[c][d] = 0;
@@ -540,14 +553,7 @@ int Engine::rebuild() {
                 }
                 continue;
             }
-            if (marched(s, d, mixed)) {
-                march_nmax_[s][d] = std::max(march_nmax_[s][d], p.n[d]);
-                const long long lines = p.N / p.n[d];
-                const int group = d == 0 ? kXLines : kMarchLines;
-                for (int g = 0; (long long)g * group < lines; ++g)
-                    march[s][d].push_back({id, g, 0, 0});
-                continue;
-            }
+            if (marched(s, d, mixed)) continue;  // below
             for (int tc = 0; tc < kInvTileClasses; ++tc) {
                 InvTileDims t = inviscid_tile(d, mixed, tc == 0 ? 32 : 64);
                 auto &L = inv[s][d][tc];
@@ -579,8 +585,48 @@ int Engine::rebuild() {
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d)
             for (int tc = 0; tc < kInvTileClasses; ++tc) append(inv[s][d][tc], r_inv_[s][d][tc]);
+    const int pin = pinned_sweep(mixed);
     for (int s = 0; s < kSchemes; ++s)
-        for (int d = 0; d < 3; ++d) append(march[s][d], r_march_[s][d]);
+        for (int d = 0; d < 3; ++d) {
+            int &chosen = inv_variant[s][d], nmin = INT_MAX, nmax = 0;
+            long long units[kInvVariants] = {};  // chunks of each variant
+            std::vector<int> ids;
+            for (size_t i = 0; i < boxes_.size() && marched(s, d, mixed); ++i) {
+                const EngineBox &b = boxes_[i];
+                if (!b.live || !b.dev.active || b.dev.p.scheme[d] != s) continue;
+                ids.push_back((int)i);
+                nmin = std::min(nmin, b.dev.p.n[d]);
+                nmax = std::max(nmax, b.dev.p.n[d]);
+                for (int v = 0; v < kInvVariants; ++v)
+                    units[v] += march_groups(b.dev.p, d) * ceil_div(b.dev.p.n[d], march_cells(d, v));
+            }
+            // lines of one length: a list of the groups serves every variant
+            // (an x sweep's chunks are a grid dimension of at most 65535)
+            march_n_[s][d] =
+                nmin == nmax && ceil_div(nmax, march_cells(d, 0)) <= 65535 ? nmax : 0;
+            Range shared;
+            for (int v = kInvVariants - 1; v >= 0; --v) {
+                Range &r = r_march_[s][d][v];
+                r = Range();
+                const bool listed = chosen >= 0 ? v == chosen
+                                                : v == pin || v + 1 == kInvVariants ||
+                                                      units[v + 1] < kChunkUnits;
+                if (!listed || ids.empty()) continue;
+                if (shared.n > 0) {
+                    r = shared;
+                    continue;
+                }
+                r.off = all.size();
+                for (int id : ids) {
+                    const BoxParams &p = boxes_[id].dev.p;
+                    const int end = march_n_[s][d] ? 1 : p.n[d];
+                    for (int c = 0; c < end; c += march_cells(d, v))
+                        for (int g = 0; g < march_groups(p, d); ++g) all.push_back({id, g, c, 0});
+                }
+                r.n = (int)(all.size() - r.off);
+                if (march_n_[s][d]) shared = r;
+            }
+        }
     for (int d = 0; d < 3; ++d) append(thomas[d], r_thomas_[d]);
     for (int c = 0; c < kLineSchemes; ++c)
         for (int d = 0; d < 3; ++d) append(cr[c][d], r_cr_[c][d]);
@@ -747,13 +793,15 @@ cudaError_t Engine::launch_lines(int d, int in, int prim_mode, cudaStream_t st) 
 
 template <typename B>
 cudaError_t Engine::launch_sweep(int s, int d, int v, int in, int prim_mode, cudaStream_t st) {
-    const Range &m = r_march_[s][d];
-    if (m.n > 0 && d == 0)
-        return launch_xsweep(s, d_boxes_, d_items_ + m.off, m.n, march_nmax_[s][d], in,
-                             kXTiles[v], prim_mode, st);
-    if (m.n > 0)
-        return launch_march(s, d, d_boxes_, d_items_ + m.off, m.n, march_nmax_[s][d], in,
-                            kMarchLen[v], st);
+    if (marched(s, d, sizeof(B) == 4)) {
+        v = std::max(v, 0);
+        const Range &m = r_march_[s][d][v];
+        const int chunks = march_n_[s][d] ? ceil_div(march_n_[s][d], march_cells(d, v)) : 1;
+        if (d == 0)
+            return launch_xsweep(s, d_boxes_, d_items_ + m.off, m.n, chunks, in, kXTiles[v],
+                                 prim_mode, st);
+        return launch_march(s, d, d_boxes_, d_items_ + m.off, m.n, chunks, in, kMarchLen[v], st);
+    }
     const Range &r = r_inv_[s][d][v < 0 ? 0 : inv_tile_class(v)];
     return launch_inviscid<B>(s, d, v, d_boxes_, d_items_ + r.off, r.n, in, d > 0, prim_mode, st);
 }
@@ -825,24 +873,14 @@ int Engine::autotune() {
         invalidate_graph();
     }
     if (!need_sweep && !need_pencil) return NUC3D_OK;
-    // NUC3D_SWEEP_RUN=1|2|4 pins the run length (32-cell tiles; with
-    // NUC3D_SWEEP_TILE=64, runs of 2 or 4 on 64-cell tiles) and
-    // NUC3D_PENCIL_DEPTH=2|4|8|16|32|64 the pencil depth (reproducibility studies)
-    if (need_sweep) {
-        if (const char *pin = std::getenv("NUC3D_SWEEP_RUN")) {
-            const int run = std::atoi(pin);
-            const char *tile = std::getenv("NUC3D_SWEEP_TILE");
-            const int tc = tile && std::atoi(tile) == 64 && run != 1 && !mixed_tiles_only32()
-                               ? 64
-                               : 32;
-            int v = 2;
-            for (int k = 0; k < kInvVariants; ++k)
-                if (kInvRunLen[k] == run && kInvTileCells[k] == tc) v = k;
-            for (int s = 0; s < kSchemes; ++s)
-                for (int d = 0; d < 3; ++d)
-                    if (has_sweep(s, d) && inv_variant[s][d] < 0) inv_variant[s][d] = v;
-            need_sweep = false;
-        }
+    const bool mixed = precision_ == NUC3D_MIXED;
+    const int pin_sweep = pinned_sweep(mixed);
+    if (need_sweep && pin_sweep >= 0) {
+        for (int s = 0; s < kSchemes; ++s)
+            for (int d = 0; d < 3; ++d)
+                if (has_sweep(s, d) && inv_variant[s][d] < 0)
+                    inv_variant[s][d] = has_list(s, d, pin_sweep) ? pin_sweep : kInvVariants - 1;
+        need_sweep = false;
     }
     bool tune_pencil = need_pencil;
     if (need_pencil) {
@@ -860,7 +898,6 @@ int Engine::autotune() {
     cudaEvent_t e0, e1;
     ECK(cudaEventCreate(&e0));
     ECK(cudaEventCreate(&e1));
-    const bool mixed = precision_ == NUC3D_MIXED;
     int rc = NUC3D_OK;
     // ms of one warm-up-then-3-repeats timing of go(), or a negative value
     // (with the error recorded) when a launch fails
@@ -882,12 +919,11 @@ int Engine::autotune() {
     for (int s = 0; s < kSchemes && rc == NUC3D_OK && need_sweep; ++s)
         for (int d = 0; d < 3 && rc == NUC3D_OK; ++d) {
             if (!has_sweep(s, d) || inv_variant[s][d] >= 0) continue;
-            int best = 0;
+            int best = -1;
             for (int v = 0; v < kInvVariants && rc == NUC3D_OK; ++v) {
-                if (inv_tile_class(v) == 1 && mixed_tiles_only32()) {
-                    inv_tune_ms[s][d][v] = 0.0;
+                inv_tune_ms[s][d][v] = 0.0;
+                if (!has_list(s, d, v) || (inv_tile_class(v) == 1 && mixed_tiles_only32()))
                     continue;
-                }
                 // the x sweep is timed as the step runs it, recovering the
                 // primitives of its tiles (prim_mode 1): it rewrites W with
                 // bitwise the values k_prim has just written
@@ -897,7 +933,7 @@ int Engine::autotune() {
                                  : launch_sweep<double>(s, d, v, 0, pm, stream_);
                 });
                 inv_tune_ms[s][d][v] = ms;
-                if (ms < inv_tune_ms[s][d][best]) best = v;
+                if (best < 0 || ms < inv_tune_ms[s][d][best]) best = v;
             }
             inv_variant[s][d] = best;
         }

@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -156,11 +157,26 @@ private:
     };
     Range r_prim_;
     Range r_inv_[kSchemes][3][kInvTileClasses];  // [scheme id][dir][32/64-cell tiles]
-    // marched pairs (marched()): one list of line groups whatever the chunk
-    // length, and the longest line of each launch
-    Range r_march_[kSchemes][3];
-    int march_nmax_[kSchemes][3] = {};
-    bool has_sweep(int s, int d) const { return r_inv_[s][d][0].n > 0 || r_march_[s][d].n > 0; }
+    // marched pairs (marched()): the work items of each variant, and the length
+    // that its boxes' lines share (items are line groups, one list for all
+    // variants) or 0 (lines of several lengths: items are the groups' chunks,
+    // so that a long box adds no empty ones to the others).  A variant
+    // has a list if it may be the pair's best: the chosen one alone once there is
+    // one, else the longest chunks and the next shorter ones while the longer
+    // make fewer than kChunkUnits (eight waves of 148 SMs x 4 units, whose tail
+    // costs less than the shorter chunks' extra overlap)
+    static constexpr long long kChunkUnits = 8 * 148 * 4;
+    Range r_march_[kSchemes][3][kInvVariants];
+    int march_n_[kSchemes][3] = {};
+    bool has_sweep(int s, int d) const {
+        for (int v = 0; v < kInvVariants; ++v)
+            if (has_list(s, d, v)) return true;
+        return false;
+    }
+    // variant v of the pair can be launched on this batch's boxes
+    bool has_list(int s, int d, int v) const {
+        return r_inv_[s][d][inv_tile_class(v)].n > 0 || r_march_[s][d][v].n > 0;
+    }
     // line groups of the CRWENO5 sweeps that march (thomas_lines_of)
     Range r_thomas_[3];
     bool any_thomas() const { return r_thomas_[1].n > 0 || r_thomas_[2].n > 0; }

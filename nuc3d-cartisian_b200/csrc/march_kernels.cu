@@ -124,8 +124,8 @@ struct Window {
     }
 };
 
-// y (DIR 1) and z (DIR 2) sweeps.  Work item (box, line group); the launch's
-// unit u is chunk u / nitems of item u % nitems.  Lines are numbered i + nx k
+// y (DIR 1) and z (DIR 2) sweeps.  Work item (box, line group, first cell); the
+// launch's unit u is chunk u / nitems of item u % nitems.  Lines are numbered i + nx k
 // (y) or i + nx j (z), so a group's lanes read consecutive addresses (y: up to
 // a row end) whatever the box's extents, and only the box's last group has
 // idle lanes.  Cells arrive in phases of four through a double buffer in
@@ -234,15 +234,16 @@ __device__ __forceinline__ void march_item(const BoxDev &bd, int group, int c0, 
 template <int SCHEME, int DIR>
 __global__ void __launch_bounds__(kThreads, 1)
     k_march(const BoxDev *__restrict__ boxes, const WorkItem *__restrict__ items, int nitems,
-            int units, int in_slot, int len) {
+            int chunks, int in_slot, int len) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int team = threadIdx.x / kTeam;
     MarchSmem &sm = reinterpret_cast<MarchSmem *>(smem_raw)[team];
-    for (int u = team * gridDim.x + blockIdx.x; u < units; u += kTeams * gridDim.x) {
+    for (int u = team * gridDim.x + blockIdx.x; u < nitems * chunks;
+         u += kTeams * gridDim.x) {
         const WorkItem it = items[u % nitems];
-        const int c0 = (u / nitems) * len;
+        const int c0 = it.b + (u / nitems) * len;
         const BoxDev &bd = boxes[it.box];
-        if (!bd.active || c0 >= bd.p.n[DIR]) continue;
+        if (!bd.active) continue;
         if (bd.p.riemann == RIEMANN_LF)
             march_item<SCHEME, DIR, true>(bd, it.a, c0, in_slot, len, team, sm);
         else
@@ -270,11 +271,11 @@ cudaError_t prepare_march_kernels() {
 }
 
 cudaError_t launch_march(int scheme, int dir, const BoxDev *boxes, const WorkItem *items,
-                         int nitems, int nmax, int in_slot, int len, cudaStream_t st) {
+                         int nitems, int chunks, int in_slot, int len, cudaStream_t st) {
     if (nitems <= 0) return cudaSuccess;
-    const int units = nitems * ((nmax + len - 1) / len);
     const March k = scheme == SCHEME_JS ? march_kernel<SCHEME_JS>(dir) : march_kernel<SCHEME_Z>(dir);
-    k<<<units < kSMs ? units : kSMs, kThreads, kSmem, st>>>(boxes, items, nitems, units, in_slot,
+    const int units = nitems * chunks;
+    k<<<units < kSMs ? units : kSMs, kThreads, kSmem, st>>>(boxes, items, nitems, chunks, in_slot,
                                                            len);
     return cudaGetLastError();
 }

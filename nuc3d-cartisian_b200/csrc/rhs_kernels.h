@@ -147,16 +147,15 @@ cudaError_t launch_inviscid(int scheme, int dir, int variant, const BoxDev *boxe
                             const WorkItem *items, int nitems, int in_slot, int accumulate,
                             int prim_mode, cudaStream_t st);
 // Marching y and z sweeps (march_kernels.cu) of the FP64 WENO5-JS / WENO5-Z
-// pairs: a work item is (box, group of 32 lines), the launch walks each line
-// in chunks of `len` cells (nmax: the longest line among the launch's boxes)
-// and adds to the RHS accumulator.  The autotuner's variant v of such a pair
+// pairs: a work item is (box, group of 32 lines, first cell), walked in `chunks`
+// chunks of `len` cells, which add to the RHS accumulator.  The autotuner's variant v of such a pair
 // is the chunk length kMarchLen[v]: short chunks give small boxes enough
 // teams, long ones re-read less of the chunk's 6-cell overlap (256^3 z: 8 to
 // 128 cells 0.95, 0.78, 0.67, 0.60, 0.57 ms; 97 x 61 x 45: 22, 20, 22, 26, 26 us).
 constexpr int kMarchLen[kInvVariants] = {8, 16, 32, 64, 128};
 // The FP64 x sweeps of weno5js, weno5z and weno7js (xsweep_kernels.cu): a work
-// item is (box, group of 16 lines), a block walks `tiles` tiles of 32 cells;
-// variant v: kXTiles[v].
+// item is (box, group of 16 lines, first cell), walked in `chunks` chunks of
+// `tiles` tiles of 32 cells, a block each; variant v: kXTiles[v].
 constexpr int kXTiles[kInvVariants] = {1, 2, 4, 8, 16};
 constexpr int kMarchLines = 32, kXLines = 16;
 constexpr bool marched(int scheme, int dir, bool mixed) {
@@ -167,14 +166,19 @@ constexpr bool marched(int scheme, int dir, bool mixed) {
 constexpr int march_cells(int dir, int variant) {
     return dir == 0 ? 32 * kXTiles[variant] : kMarchLen[variant];
 }
+// a box's line groups along d
+inline int march_groups(const BoxParams &p, int dir) {
+    const int group = dir == 0 ? kXLines : kMarchLines;
+    return (int)((p.N / p.n[dir] + group - 1) / group);
+}
 cudaError_t prepare_xsweep_kernels();
 cudaError_t launch_xsweep(int scheme, const BoxDev *boxes, const WorkItem *items, int nitems,
-                          int nmax, int in_slot, int tiles, int prim_mode, cudaStream_t st);
+                          int chunks, int in_slot, int tiles, int prim_mode, cudaStream_t st);
 cudaError_t prepare_march_kernels();
 cudaError_t launch_march(int scheme, int dir, const BoxDev *boxes, const WorkItem *items,
-                         int nitems, int nmax, int in_slot, int len, cudaStream_t st);
+                         int nitems, int chunks, int in_slot, int len, cudaStream_t st);
 // Bounded FP64 CRWENO5 sweeps along y and z by one thread per line and equation
-// (thomas_kernels.cu): work items as launch_march's.  free_slot: the state slot
+// (thomas_kernels.cu): work items (box, group of 32 lines).  free_slot: the state slot
 // that is neither u_n nor in_slot; the boxes' viscous fluxes and that slot are
 // scratch, so the viscous fluxes are computed after these sweeps.
 constexpr bool thomas_lines_of(int scheme, int dir, bool mixed, bool bounded) {

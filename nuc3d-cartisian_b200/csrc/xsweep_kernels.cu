@@ -140,7 +140,8 @@ struct XGeom {
 
 }  // namespace
 
-// Work item (box, group of 16 lines); blockIdx.y: the chunk of `tiles` tiles.
+// Work item (box, group of 16 lines, first cell); blockIdx.y: the chunk of `tiles`
+// tiles from there.
 // The primitives are recovered from the state and W is written for the tile's
 // own cells; PM 2: their eigenvalues are folded into the box's maxima as well.
 template <int SCHEME, int PM>
@@ -156,8 +157,8 @@ __global__ void __launch_bounds__(kThreads, SCHEME == SCHEME_W7 ? 3 : 4)
     const BoxDev &bd = boxes[it.box];
     const BoxParams &bp = bd.p;
     const int n = bp.n[0];
-    const int first = blockIdx.y * tiles * TC;
-    if (!bd.active || first >= n) return;
+    const int first = it.b + blockIdx.y * tiles * TC;
+    if (!bd.active) return;
     const long long np = bd.np;
     const int nlines = bp.n[1] * bp.n[2], L0 = it.a * TL;
     const double *const qbase = fieldU(bd, in_slot, 0);
@@ -306,12 +307,11 @@ cudaError_t prepare_xsweep_kernels() {
 }
 
 cudaError_t launch_xsweep(int scheme, const BoxDev *boxes, const WorkItem *items, int nitems,
-                          int nmax, int in_slot, int tiles, int prim_mode, cudaStream_t st) {
+                          int chunks, int in_slot, int tiles, int prim_mode, cudaStream_t st) {
     if (nitems <= 0) return cudaSuccess;
     size_t smem;
     const XSweep k = xsweep_kernel(scheme, prim_mode, smem);
-    const dim3 grid(nitems, (nmax + tiles * TC - 1) / (tiles * TC));
-    k<<<grid, kThreads, smem, st>>>(boxes, items, in_slot, tiles);
+    k<<<dim3(nitems, chunks), kThreads, smem, st>>>(boxes, items, in_slot, tiles);
     return cudaGetLastError();
 }
 

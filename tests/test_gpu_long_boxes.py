@@ -8,7 +8,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("axis,long", [("z", 1 << 20)])
+@pytest.mark.parametrize("axis,long", [("z", 1 << 20), ("x", 1 << 21)])
 def test_long_box_repeats_short_one(axis, long):
     import torch
     import nuc3d_b200 as nb
