@@ -262,7 +262,8 @@ __global__ void k_export_flags(FlagPtrs f, unsigned *out) {
 
 Engine::Engine(int precision, cudaStream_t stream) : precision_(precision), stream_(stream) {
     cudaGetDevice(&device_);
-    for (auto &p : pencil_of_class) std::fill(p, p + kPencilClasses, (signed char)-1);
+    std::memset(pencil_of_class, -1, sizeof pencil_of_class);
+    std::memset(variant_of_class_, -1, sizeof variant_of_class_);
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -589,16 +590,22 @@ int Engine::rebuild() {
     for (int s = 0; s < kSchemes; ++s)
         for (int d = 0; d < 3; ++d) {
             int &chosen = inv_variant[s][d], nmin = INT_MAX, nmax = 0;
-            long long units[kInvVariants] = {};  // chunks of each variant
+            long long units[kInvVariants] = {}, cells = 0;  // chunks of each variant
             std::vector<int> ids;
             for (size_t i = 0; i < boxes_.size() && marched(s, d, mixed); ++i) {
                 const EngineBox &b = boxes_[i];
                 if (!b.live || !b.dev.active || b.dev.p.scheme[d] != s) continue;
                 ids.push_back((int)i);
+                cells += b.dev.p.N;
                 nmin = std::min(nmin, b.dev.p.n[d]);
                 nmax = std::max(nmax, b.dev.p.n[d]);
                 for (int v = 0; v < kInvVariants; ++v)
                     units[v] += march_groups(b.dev.p, d) * ceil_div(b.dev.p.n[d], march_cells(d, v));
+            }
+            if (!ids.empty()) {
+                variant_slot_[s][d] = &variant_of_class_[s][d][nmax < 32 ? 0 : (nmax < 128 ? 1 : 2)]
+                                                        [size_class(cells)];
+                chosen = *variant_slot_[s][d];
             }
             // lines of one length: a list of the groups serves every variant
             // (an x sweep's chunks are a grid dimension of at most 65535)
@@ -848,11 +855,23 @@ int Engine::enqueue_step(cudaStream_t s) {
     return precision_ == NUC3D_MIXED ? enqueue_step_t<float>(s) : enqueue_step_t<double>(s);
 }
 
+int Engine::size_class(long long cells) {
+    int c = 0;
+    while (c + 1 < kSizeClasses && (cells >> (2 * (c + 1))) > 0) ++c;
+    return c;
+}
+
+void Engine::keep_variant(int s, int d, int v) {
+    inv_variant[s][d] = v;
+    if (marched(s, d, precision_ == NUC3D_MIXED)) *variant_slot_[s][d] = (signed char)v;
+}
+
 // Picks the variant of the directional sweep per scheme and direction, and the
-// pencil depth of the 2.5-D stencil kernels, by timing every variant on this
-// batch's own work lists: the sweeps on the first step after a rebuild that
-// brings a new (scheme, direction) pair, the depth on the first step in each
-// power of four of active cells.  The sweeps only write the RHS accumulator (and the x
+// pencil depth of the 2.5-D stencil kernels, by timing the variants on this
+// batch's own work lists: a sweep on the first step with a new (scheme, direction)
+// pair, a marched one again at each size not met before (variant_of_class_), the
+// depth on the first step in each power of four of active cells.  The sweeps
+// only write the RHS accumulator (and the x
 // sweep the primitives, with the values they already hold) and the
 // viscous-flux kernel the viscous fluxes, which every stage recomputes; the
 // update is timed as a first stage, which writes only the u1 slot that the
@@ -864,9 +883,7 @@ int Engine::autotune() {
         for (int d = 0; d < 3; ++d)
             need_sweep = need_sweep || (has_sweep(s, d) && inv_variant[s][d] < 0);
     const bool stencils = r_25d_[0][0].n > 0 || r_25d_[1][0].n > 0;
-    int cls = 0;  // size class: floor(log4(active cells))
-    while (cls + 1 < kPencilClasses && (active_cells_ >> (2 * (cls + 1))) > 0) ++cls;
-    signed char &kept_pencil = pencil_of_class[short_pencils_][cls];
+    signed char &kept_pencil = pencil_of_class[short_pencils_][size_class(active_cells_)];
     const bool need_pencil = stencils && kept_pencil < 0;
     if (stencils && !need_pencil && pencil_variant != kept_pencil) {
         pencil_variant = kept_pencil;
@@ -879,7 +896,7 @@ int Engine::autotune() {
         for (int s = 0; s < kSchemes; ++s)
             for (int d = 0; d < 3; ++d)
                 if (has_sweep(s, d) && inv_variant[s][d] < 0)
-                    inv_variant[s][d] = has_list(s, d, pin_sweep) ? pin_sweep : kInvVariants - 1;
+                    keep_variant(s, d, has_list(s, d, pin_sweep) ? pin_sweep : kInvVariants - 1);
         need_sweep = false;
     }
     bool tune_pencil = need_pencil;
@@ -935,7 +952,7 @@ int Engine::autotune() {
                 inv_tune_ms[s][d][v] = ms;
                 if (best < 0 || ms < inv_tune_ms[s][d][best]) best = v;
             }
-            inv_variant[s][d] = best;
+            keep_variant(s, d, best);
         }
     if (tune_pencil && rc == NUC3D_OK) {
         int best = 0;

@@ -75,7 +75,7 @@ public:
     int profile_flush();
     // autotuned sweep variant (tile length and run length, kInvTileCells /
     // kInvRunLen) per [scheme JS/Z/-/W7][dir] (-1: not tuned yet) and the
-    // measured milliseconds per launch of each variant
+    // milliseconds per launch of each variant when it was last timed (0: not)
     int inv_variant[kSchemes][3] = {{-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1},
                                     {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1},
                                     {-1, -1, -1}, {-1, -1, -1}, {-1, -1, -1}};
@@ -96,8 +96,8 @@ public:
     // takes that class's depth)
     int pencil_variant = -1;
     double pencil_tune_ms[kPencils] = {};
-    static constexpr int kPencilClasses = 20;
-    signed char pencil_of_class[2][kPencilClasses];
+    static constexpr int kSizeClasses = 20;  // floor(log4(cells))
+    signed char pencil_of_class[2][kSizeClasses];
 
     static long long box_bytes(const nuc3d_box_desc &d);
     static int validate(const nuc3d_box_desc &d, std::string *why);
@@ -124,6 +124,9 @@ private:
     cudaError_t launch_update_classes(int v, StageArgs sa, cudaStream_t st);
     void invalidate_graph();
     int autotune();
+    static int size_class(long long cells);
+    // the pair's variant from now on (marched pairs: at this size)
+    void keep_variant(int s, int d, int v);
 
     // Device memory of this engine comes from its own stream-ordered pool, which
     // keeps up to kPoolKeep bytes of what it frees (the next box or spectra call
@@ -168,6 +171,12 @@ private:
     static constexpr long long kChunkUnits = 8 * 148 * 4;
     Range r_march_[kSchemes][3][kInvVariants];
     int march_n_[kSchemes][3] = {};
+    // The variant found for each power of four of a marched pair's cells and for
+    // lines below 32, below 128 and longer: the best chunk grows with both (see
+    // kMarchLen), so what small boxes were tuned to does not stay for large ones.
+    // -1: not tuned yet.  variant_slot_: the current batch's entry.
+    signed char variant_of_class_[kSchemes][3][3][kSizeClasses];
+    signed char *variant_slot_[kSchemes][3] = {};
     bool has_sweep(int s, int d) const {
         for (int v = 0; v < kInvVariants; ++v)
             if (has_list(s, d, v)) return true;
