@@ -499,12 +499,20 @@ int Engine::rebuild() {
     const int crtl = crweno_tile_lines();
     for (int c = 0; c < kLineSchemes; ++c)
         for (int d = 0; d < 3; ++d) cr_nmax_[c][d] = cr_ms_[c][d] = 0;
-    // (blocks of the 2.5-D kernels at 16 planes)
-    long long blocks16 = 0;
+    // tiles of the 2.5-D kernels, their planes (at most 64 each) and the blocks that
+    // 16 planes make
+    long long tiles = 0, planes = 0, blocks16 = 0;
     for (const EngineBox &b : boxes_)
-        if (b.live && b.dev.active)
-            blocks16 += (long long)ceil_div(b.dev.p.n[0], kT25X) * ceil_div(b.dev.p.n[1], kT25Y) *
-                        ceil_div(b.dev.p.n[2], 16);
+        if (b.live && b.dev.active) {
+            const int *n = b.dev.p.n;
+            const long long t = (long long)ceil_div(n[0], kT25X) * ceil_div(n[1], kT25Y);
+            tiles += t;
+            planes += t * std::min(n[2], 64);
+            blocks16 += t * ceil_div(n[2], 16);
+        }
+    plane_class_ = 0;
+    while (plane_class_ + 1 < kPlaneClasses && planes >= tiles * (16LL << plane_class_))
+        ++plane_class_;
     short_pencils_ = blocks16 <= kPencilShortBlocks || pinned_pencil() >= kLongPencils;
     any_visc_ = false;
     nactive_ = 0;
@@ -870,7 +878,7 @@ void Engine::keep_variant(int s, int d, int v) {
 // pencil depth of the 2.5-D stencil kernels, by timing the variants on this
 // batch's own work lists: a sweep on the first step with a new (scheme, direction)
 // pair, a marched one again at each size not met before (variant_of_class_), the
-// depth on the first step in each power of four of active cells.  The sweeps
+// depth on the first step in each class of pencil_of_class.  The sweeps
 // only write the RHS accumulator (and the x
 // sweep the primitives, with the values they already hold) and the
 // viscous-flux kernel the viscous fluxes, which every stage recomputes; the
@@ -883,7 +891,8 @@ int Engine::autotune() {
         for (int d = 0; d < 3; ++d)
             need_sweep = need_sweep || (has_sweep(s, d) && inv_variant[s][d] < 0);
     const bool stencils = r_25d_[0][0].n > 0 || r_25d_[1][0].n > 0;
-    signed char &kept_pencil = pencil_of_class[short_pencils_][size_class(active_cells_)];
+    signed char &kept_pencil =
+        pencil_of_class[short_pencils_][plane_class_][size_class(active_cells_)];
     const bool need_pencil = stencils && kept_pencil < 0;
     if (stencils && !need_pencil && pencil_variant != kept_pencil) {
         pencil_variant = kept_pencil;

@@ -90,14 +90,16 @@ public:
     }
     // autotuned pencil depth of the 2.5-D stencil kernels: index into
     // kPencilDepths (-1: not tuned yet), the measured milliseconds of one
-    // viscous-flux + update pass per depth of the last tuning, and the depth
-    // found for each power of four of active cells with and without the short
-    // depths (a batch that grows or shrinks into a size class it has been in
-    // takes that class's depth)
+    // viscous-flux + update pass per depth of the last tuning (0: not timed), and
+    // the depth found for each power of four of active cells, with and without
+    // the short depths and for each power of two of the tiles' mean planes up to
+    // 64 (flat boxes cannot tell the depths beyond their own extent apart).  A
+    // batch that grows or shrinks into a class it has been in takes its depth.
     int pencil_variant = -1;
     double pencil_tune_ms[kPencils] = {};
     static constexpr int kSizeClasses = 20;  // floor(log4(cells))
-    signed char pencil_of_class[2][kSizeClasses];
+    static constexpr int kPlaneClasses = 4;  // 8, 16, 32, 64 planes and more
+    signed char pencil_of_class[2][kPlaneClasses][kSizeClasses];
 
     static long long box_bytes(const nuc3d_box_desc &d);
     static int validate(const nuc3d_box_desc &d, std::string *why);
@@ -199,6 +201,7 @@ private:
     // kPencilDepths]; the short depths' lists only where short_pencils_
     Range r_25d_[kVisClasses][kPencils];
     bool short_pencils_ = false;
+    int plane_class_ = 0;
     long long active_cells_ = 0;
     // blocks up to which the short pencils are worth timing: two waves of 148
     // SMs x 2 blocks at depth 16

@@ -27,3 +27,23 @@ def test_chunks_are_chosen_again_for_a_large_box():
         for name, (choice, _) in b.tuning().items():
             if name in first:
                 assert choice == first[name][0]
+
+
+def test_pencil_depth_of_a_flat_batch_does_not_stay_for_a_tall_one():
+    import nuc3d_b200 as nb
+    with nb.Batch(nb.FP64) as b:
+        # both have more than 600 tiles of 16 planes and 2^20 .. 2^22 cells
+        flat = b.add(nb.BoxDesc(512, 512, 8, mach=0.3))
+        b.init_state(flat, "tgv")
+        b.step(1)
+        of_flat = b.tuning()["pencil_depth"]
+        tall = b.add(nb.BoxDesc(128, 128, 160, mach=0.3))
+        b.init_state(tall, "tgv")
+        b.set_active(flat, False)
+        b.step(1)
+        of_tall = b.tuning()["pencil_depth"]
+        assert of_tall[1] != of_flat[1]  # timed on its own
+        b.set_active(flat, True)
+        b.set_active(tall, False)
+        b.step(1)
+        assert b.tuning()["pencil_depth"][0] == of_flat[0]
