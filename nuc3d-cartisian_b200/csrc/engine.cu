@@ -216,6 +216,58 @@ struct CopyLane {
 std::mutex g_lane_mu;
 std::map<int, CopyLane> g_lanes[2];  // [upload, download][device]
 
+// Device memory of the engines on one device comes from a pool that they share,
+// made by the first of them and destroyed with the last.  It keeps up to kKeep
+// bytes of what they free, all engines together, so that the next box or spectra
+// call maps no memory; an allocation that fails gives these back and tries
+// again.  (A pool per engine held kKeep each, and a new engine mapped memory
+// that the process had just freed: creating a 32^3 solver beside another took
+// 0.7 ms, in the shared pool as in CUDA's own 0.12.)  The release threshold counts
+// what is in use too, so it follows the boxes' bytes.
+struct DevicePool {
+    static constexpr unsigned long long kKeep = 256ull << 20;
+    cudaMemPool_t pool = nullptr;
+    int engines = 0;
+    unsigned long long box_bytes = 0;
+};
+std::mutex g_pool_mu;
+std::map<int, DevicePool> g_pools;
+
+// the boxes of the device's engines have grown by `bytes` (shrunk: negative)
+void pool_boxes(DevicePool &p, long long bytes) {
+    p.box_bytes += bytes;
+    unsigned long long keep = p.box_bytes + DevicePool::kKeep;
+    if (p.pool) cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+void pool_boxes(int device, long long bytes) {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    pool_boxes(g_pools[device], bytes);
+}
+cudaMemPool_t pool_join(int device) {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    DevicePool &p = g_pools[device];
+    if (p.engines++ == 0) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        if (cudaMemPoolCreate(&p.pool, &props) != cudaSuccess) {
+            p.pool = nullptr;
+            cudaGetLastError();
+        }
+        pool_boxes(p, 0);
+    }
+    return p.pool;
+}
+// (everything the engine allocated has been freed and its stream waited for)
+void pool_leave(int device) {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    DevicePool &p = g_pools[device];
+    if (--p.engines > 0) return;
+    if (p.pool) cudaMemPoolDestroy(p.pool);
+    p.pool = nullptr;
+}
+
 // NUC3D_STEP_FORK=0 keeps a captured step on one stream (the viscous fluxes
 // then run between the x and y sweeps); the default forks them
 bool step_fork_enabled() {
@@ -264,26 +316,18 @@ Engine::Engine(int precision, cudaStream_t stream) : precision_(precision), stre
     cudaGetDevice(&device_);
     std::memset(pencil_of_class, -1, sizeof pencil_of_class);
     std::memset(variant_of_class_, -1, sizeof variant_of_class_);
-    cudaMemPoolProps props{};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = device_;
-    if (cudaMemPoolCreate(&pool_, &props) != cudaSuccess) {
-        pool_ = nullptr;
-        cudaGetLastError();
-    }
-    set_pool_keep();
-}
-
-void Engine::set_pool_keep() {
-    if (!pool_) return;
-    unsigned long long keep = box_bytes_ + kPoolKeep;
-    cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &keep);
+    pool_ = pool_join(device_);
 }
 
 cudaError_t Engine::device_alloc(void **p, size_t bytes) {
-    return pool_ ? cudaMallocFromPoolAsync(p, bytes, pool_, stream_)
-                 : cudaMallocAsync(p, bytes, stream_);
+    if (!pool_) return cudaMallocAsync(p, bytes, stream_);
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool_, stream_);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        cudaMemPoolTrimTo(pool_, 0);  // what the pool keeps idle
+        e = cudaMallocFromPoolAsync(p, bytes, pool_, stream_);
+    }
+    return e;
 }
 
 Engine::~Engine() {
@@ -306,7 +350,9 @@ Engine::~Engine() {
     if (d_stats_) cudaFreeAsync(d_stats_, stream_);
     cudaStreamSynchronize(stream_);
     spectra_plan_.release();
-    if (pool_) cudaMemPoolDestroy(pool_);
+    for (auto &b : boxes_)
+        if (b.live) pool_boxes(device_, -(long long)b.bytes);
+    pool_leave(device_);
     for (cudaEvent_t e : ev_pool_) cudaEventDestroy(e);
     for (cudaEvent_t e : copy_ev_)
         if (e) cudaEventDestroy(e);
@@ -388,8 +434,7 @@ int Engine::add_box(const nuc3d_box_desc &d, int *id) {
     }
     *id = slot;
     dirty_ = true;
-    box_bytes_ += b.bytes;
-    set_pool_keep();
+    pool_boxes(device_, (long long)b.bytes);
     return NUC3D_OK;
 }
 
@@ -399,8 +444,7 @@ int Engine::remove_box(int id) {
     EngineBox &b = boxes_[id];
     ECK(cudaFreeAsync(b.mem, stream_));
     if (b.force_mem) ECK(cudaFreeAsync(b.force_mem, stream_));
-    box_bytes_ -= b.bytes;
-    set_pool_keep();
+    pool_boxes(device_, -(long long)b.bytes);
     b = EngineBox();
     dirty_ = true;
     return NUC3D_OK;

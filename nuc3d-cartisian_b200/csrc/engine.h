@@ -130,19 +130,14 @@ private:
     // the pair's variant from now on (marched pairs: at this size)
     void keep_variant(int s, int d, int v);
 
-    // Device memory of this engine comes from its own stream-ordered pool, which
-    // keeps up to kPoolKeep bytes of what it frees (the next box or spectra call
-    // then maps no memory) and is destroyed with the engine.  The pool's release
-    // threshold counts what is in use too, so it follows the boxes' bytes.
-    static constexpr unsigned long long kPoolKeep = 256ull << 20;
-    unsigned long long box_bytes_ = 0;
-    void set_pool_keep();
+    // stream-ordered device memory from the pool that the engines of a device
+    // share (DevicePool, engine.cu)
     cudaError_t device_alloc(void **p, size_t bytes);
     template <typename T>
     cudaError_t device_alloc(T **p, size_t bytes) {
         return device_alloc(reinterpret_cast<void **>(p), bytes);
     }
-    cudaMemPool_t pool_ = nullptr;
+    cudaMemPool_t pool_ = nullptr;  // null: none could be made, the default pool serves
     SpectraPlan spectra_plan_;  // of the last box size asked for
 
     int precision_;
