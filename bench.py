@@ -536,6 +536,36 @@ def run_b200(args, rank, world, local_rank):
     return line
 
 
+# what the bench's one JSON line holds; the legs' other results stand on the
+# detail line before it
+HEADLINE = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+            "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "config", "e2e",
+            "gpu_launches", "clocks")
+HEADLINE_PART = {
+    "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "steps"),
+    "roofline": ("bound", "achieved", "peak", "unit", "frac"),
+    "mixed": ("value", "ms_per_step", "rel_l2_vs_fp64"),
+    "cpu_baseline": ("value", "unit", "cores", "kind"),
+}
+
+
+def headline(line):
+    """The headline fields of a result: under 2 KB, so that a reader of the
+    output's tail gets the line whole."""
+    out = {k: line[k] for k in HEADLINE}
+    for key, part in HEADLINE_PART.items():
+        if line.get(key):
+            out[key] = {k: line[key][k] for k in part if k in line[key]}
+    return out
+
+
+def report(line):
+    """Prints every leg's results on a line of their own, then the headline as
+    the output's one JSON line."""
+    print("detail " + json.dumps(line), flush=True)
+    print(json.dumps(headline(line)), flush=True)
+
+
 def spectrum_diff(a, b):
     """Max relative difference over the shells of spectrum b that hold at
     least 1e-10 of its total."""
@@ -971,7 +1001,7 @@ def main():
         }
     line = run_b200(args, rank, world, local_rank)
     if line is not None:
-        print(json.dumps(line), flush=True)
+        report(line)
 
 
 if __name__ == "__main__":
