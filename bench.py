@@ -76,13 +76,14 @@ FLOPS_PER_CELL_STAGE = 3 * FLOPS_INV_Z + FLOPS_PRIM + 156 + 111  # + viscous flu
 FLOPS_INV_LAUNCH = FLOPS_INV_Z + FLOPS_PRIM / 3
 STATE_BYTES_PER_CELL_UPDATE = 320  # compulsory FP64 state traffic of 3 RK stages
 # DRAM bytes (read + write) per launch of the FP64 WENO5-Z sweep at 256^3,
-# mean of x, y, z: the ncu capture at 128^3 in
-# profiles/sweeps_weno5z_fp64_128.md (226.8, 274.1, 272.9 MB; the x sweep
-# reads the state only and writes the primitives as well as its RHS) scaled
-# by the cell count (x8); the traffic of a sweep is proportional to the cells
-# it covers (whole lines, no halo growth with size along the other axes).
-INV_TRAFFIC_BYTES = 8 * (226.784768e6 + 274.140928e6 + 272.945664e6) / 3
-INV_TRAFFIC_NOTE = "ncu dram__bytes_read+write of the 128^3 capture x8 (cells), mean of x/y/z"
+# mean of x, y, z, derived: the reads of the ncu capture at 128^3 in
+# profiles/sweeps_weno5z_fp64_128.md (99.8, 224.9, 224.5 MB) scaled by the cell
+# count (x8), and the compulsory writes of 256^3 (x: the RHS and six primitives,
+# 88 B per cell; y and z: the RHS, 40 B).  The capture's writes do not scale: up
+# to L2's capacity of each launch's last writes is still in L2 when it ends.
+INV_TRAFFIC_BYTES = (8 * (99.8e6 + 224.9e6 + 224.5e6) + 256 ** 3 * (88 + 40 + 40)) / 3
+INV_TRAFFIC_NOTE = ("derived: ncu dram__bytes_read of the 128^3 capture x8 (cells) and the "
+                    "compulsory writes, mean of x/y/z")
 
 
 def hbm_peak_gbs():

@@ -52,3 +52,11 @@ def test_headline_is_the_one_json_line_and_short(capsys):
         {k: line["clocks"][k] for k in ("sm_mhz", "sm_max_mhz", "reasons")}
     # the legs are all there, on the line before
     assert json.loads(out[-2].split(" ", 1)[1])["schemes"] == line["schemes"]
+
+
+def test_stated_sweep_traffic_is_not_below_the_compulsory_bytes():
+    import bench
+    # per cell: x reads the state and writes the RHS and six primitives; y and z read
+    # the state, u_n, p, c and the RHS and write the RHS
+    least = 256 ** 3 * 8 * ((5 + 11) + 2 * (5 + 3 + 5 + 5)) / 3
+    assert least <= bench.INV_TRAFFIC_BYTES < 1.25 * least
