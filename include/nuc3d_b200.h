@@ -265,9 +265,9 @@ NUC3D_API int nuc3d_probe_peak(int precision, double *tflops);
 /* Autotuner result.  The directional WENO sweep has variants in two tile
  * shapes: 32 cells along the sweep with runs of 1, 2 or 4 consecutive faces
  * per thread, and 64 cells with runs of 2 or 4 (fewer staged halo cells per
- * cell, twice the shared memory per block).  The first step after the set of
- * (scheme, direction) pairs changes times every variant on the live boxes and
- * keeps the fastest.  run_len[s*3+d] (s: the scheme id, NUC3D_WENO5JS ..
+ * cell, twice the shared memory per block).  The first step with a new (scheme,
+ * direction) pair times its variants on the live boxes and keeps the fastest.
+ * run_len[s*3+d] (s: the scheme id, NUC3D_WENO5JS ..
  * NUC3D_UPWIND1ST; d: x, y, z) receives the chosen run length (0 = not tuned;
  * always 0 for the line-solve schemes CRWENO5, hccs and hccs77, whose lines
  * have no run variants),
@@ -285,7 +285,10 @@ NUC3D_API int nuc3d_probe_peak(int precision, double *tflops);
  * walking a line in chunks instead: their five variants are the chunk lengths
  * in cells (y, z: 8, 16, 32, 64, 128; x: 32, 64, 128, 256, 512), reported as
  * both run_len and tile_cells, the milliseconds in the same order in ms (the
- * first three) and ms64 (the last two). */
+ * first three) and ms64 (the last two).  These pairs are tuned at each power of
+ * four of their cells and line length (below 32, below 128, longer) when it is
+ * first met and keep a choice for each; chunks shorter than one that already
+ * makes more than eight waves are not timed (0). */
 #define NUC3D_TUNING_SLOTS 27
 NUC3D_API int nuc3d_tuning(const nuc3d_ctx *ctx, int *run_len, double *ms);
 NUC3D_API int nuc3d_batch_tuning(const nuc3d_batch *b, int *run_len, double *ms);
@@ -294,13 +297,14 @@ NUC3D_API int nuc3d_batch_tuning_tiles(const nuc3d_batch *b, int *tile_cells, do
 /* The other autotuned shape: the pencil depth of the 2.5-D stencil kernels
  * (viscous flux, update), i.e. how many z-planes one 32 x 8 column tile
  * marches (each tile re-reads a 6-plane halo, so deeper pencils read less but
- * make fewer, longer blocks).  The first step, and every step after the
- * batch's active cells have grown or shrunk past a factor 2 of those it was
- * tuned at into a size not tuned before, times viscous-flux + update passes
- * on the live boxes and keeps the fastest depth; boxes too small to fill the
- * GPU may get 8, 4 or 2 planes.  *depth receives the chosen depth (0 = not
- * tuned), ms (NUC3D_PENCIL_DEPTHS doubles, may be NULL) the measured
- * milliseconds per pass for depths {32, 16, 64}. */
+ * make fewer, longer blocks).  The first step at each power of four of active
+ * cells (and power of two of the boxes' mean planes, up to 64) times
+ * viscous-flux + update passes on the live boxes and keeps the fastest depth for
+ * that size.  Depths: 32 and 16; 64 where 16 is slower than 32; 8, 4 and 2 where
+ * 16 planes make at most 600 blocks and each was faster than the one before.
+ * *depth receives the chosen depth (0 = not tuned), ms (NUC3D_PENCIL_DEPTHS
+ * doubles, may be NULL) the milliseconds per pass for depths {32, 16, 64} when
+ * they were last timed (0: not). */
 #define NUC3D_PENCIL_DEPTHS 3
 NUC3D_API int nuc3d_tuning_pencil(const nuc3d_ctx *ctx, int *depth, double *ms);
 NUC3D_API int nuc3d_batch_tuning_pencil(const nuc3d_batch *b, int *depth, double *ms);

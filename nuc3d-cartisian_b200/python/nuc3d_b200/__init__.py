@@ -763,8 +763,9 @@ def _spectra(fn, *args):
 
 def _tuning(fn, h, fn_pencil=None, fn_tiles=None):
     """{"<scheme>_<dir>": (chosen "<tile cells>x<run length>", {variant: ms per
-    launch}), "pencil_depth": (chosen depth, {depth: ms per viscous-flux +
-    update pass})}; the sweep variants are "32x1", "32x2", "32x4", "64x2",
+    launch, 0.0 where it was not timed}), "pencil_depth": (chosen depth, {depth:
+    ms per viscous-flux + update pass, of 32, 16 and 64 planes those timed})};
+    the sweep variants are "32x1", "32x2", "32x4", "64x2",
     "64x4" (cells per tile along the sweep x faces per thread); sweeps that
     march are named by the cells of a chunk, the FP64 WENO5-JS / WENO5-Z y and
     z sweeps "8x8" to "128x128", the FP64 WENO5 / WENO7 x sweeps "32x32" to
@@ -797,7 +798,7 @@ def _tuning(fn, h, fn_pencil=None, fn_tiles=None):
         check(fn_pencil(h, C.byref(depth), pms.ctypes.data))
         if depth.value:
             out["pencil_depth"] = (depth.value, {D: round(float(pms[v]), 4)
-                                                 for v, D in enumerate(PENCIL_DEPTHS)})
+                                                 for v, D in enumerate(PENCIL_DEPTHS) if pms[v]})
     return out
 
 
