@@ -224,7 +224,8 @@ __global__ void __launch_bounds__(kModeThreads)
     sum(0, e2[0]);
     sum(1, e2[1]);
     // shell: theta - 1 multiplies the shell's modes; band: the gain P / (2 E_b)
-    // (zero for a band without energy)
+    // (zero for a band of exactly zero energy; one that holds only rounding noise,
+    // E_b ~ 1e-33, is driven by its noise at the full rate)
     const double theta = fp.band ? 0.0 : sqrt(fabs(fp.amp - tot[1]) / tot[0]);
     const double gain = fp.band ? (tot[0] > 0.0 ? fp.amp / (2.0 * tot[0]) : 0.0) : theta - 1.0;
     double power = 0.0;

@@ -9,12 +9,14 @@
 // teams per SM takes (line group, chunk) items in turn; teams meet only at
 // their own named barriers.
 //
-// Bound: the FP64 pipe (about 86 FP64 instructions per cell and equation, 158
-// instructions in all).  A march forms each difference, square and split once
+// Bound: the FP64 pipe and the latency of its chains (about 86 FP64 instructions
+// per cell and equation, 158 instructions in all; 160^3: FP64 pipe busy 60 % of
+// the cycles, issue slots 55 %, DRAM 39 %, with the 20 warps that the registers
+// admit).  A march forms each difference, square and split once
 // per cell: a tile of 32 cells whose threads each hold a run of 2 or 4 faces
 // (k_inviscid, which these sweeps replaced) rebuilds its
 // windows for every run and stages 38 cells for 32.  256^3 WENO5-Z, per launch:
-// y 0.68 -> 0.59 ms, z 0.70 -> 0.57 ms (about 3/4 of the FP64 pipe's rate).
+// y 0.68 -> 0.59 ms, z 0.70 -> 0.57 ms.
 // Measured beside it: one warp per sign (30 warps of 64 registers) 0.89 / 0.88,
 // three teams of 128 registers 0.63 / 0.62, separate blocks of one team with
 // the loads a cell ahead in registers 0.70 / 0.70, with the double buffer 0.67.
@@ -125,15 +127,15 @@ struct Window {
 };
 
 // y (DIR 1) and z (DIR 2) sweeps.  Work item (box, line group, first cell); the
-// launch's unit u is chunk u / nitems of item u % nitems.  Lines are numbered i + nx k
-// (y) or i + nx j (z), so a group's lanes read consecutive addresses (y: up to
-// a row end) whatever the box's extents, and only the box's last group has
-// idle lanes.  Cells arrive in phases of four through a double buffer in
-// shared memory filled with cp.async a phase ahead: the '+' warps copy their
-// equation's state, the '-' warps its RHS, the first four u_n, p and c of a row
-// each.  The signs' parts meet in shared memory: the '+' warp leaves RHS + its
-// part, the '-' warp its part, and after the next phase's barrier each adds
-// and stores two of the four rows.
+// launch's unit u is chunk u / nitems of item u % nitems.  Lines are numbered
+// i + nx k (y) or i + nx j (z), so a group's lanes read consecutive addresses (y:
+// up to a row end) whatever the box's extents, and only the box's last group has
+// idle lanes.  Cells arrive in phases of four through a double buffer in shared
+// memory filled with cp.async a phase ahead: each warp copies its equation's
+// state and RHS, the first four warps the u_n, p and c of a row each.  A warp
+// carries both signs of its equation and stores its own rows, so the warps share
+// u_n, p and c alone; the team's barrier at the head of a phase says that these
+// have arrived and that the other buffer has been read.
 struct MarchSmem {
     double Q[2][5][2][4][32];  // [buffer][equation][state, RHS][row][line]
     double W[2][12][32];       // [buffer][row x (u_n, p, c)][line]

@@ -13,7 +13,8 @@
 // instructions on its partitioned solve, shared-memory rows and index work for
 // each FP64 one and is bound by instruction issue; here a row costs about 110
 // instructions forward, 82 of them FP64, and 25 back.  Bound: HBM, for the 64
-// bytes of c' and d' that each face and equation writes and reads back.  192^3:
+// bytes of c' and d' that each face and equation writes and reads back (160^3: 485
+// bytes of DRAM traffic per cell at 5.8 TB/s, FP64 pipe 31 %).  192^3:
 // y 1.01 -> 0.61 ms, z 1.02 -> 0.59 ms per launch (5.6 TB/s; 16 warps of 128
 // registers per SM with 8 faces' loads together on the way back; 20 warps of 96
 // with 4 measured 0.62 / 0.61).
