@@ -855,7 +855,7 @@ cudaError_t Engine::launch_sweep(int s, int d, int v, int in, int prim_mode, cud
     if (marched(s, d, sizeof(B) == 4)) {
         v = std::max(v, 0);
         const Range &m = r_march_[s][d][v];
-        const int chunks = march_n_[s][d] ? ceil_div(march_n_[s][d], march_cells(d, v)) : 1;
+        const int chunks = march_n_[s][d] ? ceil_div(march_n_[s][d], march_cells(d, v)) : 0;
         if (d == 0)
             return launch_xsweep(s, d_boxes_, d_items_ + m.off, m.n, chunks, in, kXTiles[v],
                                  prim_mode, st);

@@ -276,6 +276,7 @@ cudaError_t launch_march(int scheme, int dir, const BoxDev *boxes, const WorkIte
                          int nitems, int chunks, int in_slot, int len, cudaStream_t st) {
     if (nitems <= 0) return cudaSuccess;
     const March k = scheme == SCHEME_JS ? march_kernel<SCHEME_JS>(dir) : march_kernel<SCHEME_Z>(dir);
+    if (chunks == 0) chunks = 1;  // items are chunks
     const int units = nitems * chunks;
     k<<<units < kSMs ? units : kSMs, kThreads, kSmem, st>>>(boxes, items, nitems, chunks, in_slot,
                                                            len);

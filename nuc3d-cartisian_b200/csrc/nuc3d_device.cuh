@@ -30,6 +30,10 @@ enum : int {
     SCHEME_U1 = 8
 };
 
+// v, the same in all lanes, in a form that lets the compiler keep what follows from
+// it in uniform registers (called by whole warps)
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // reconstruction stencil half-width (the reference's bufferSize,
 // fieldOperator.cpp:128-175): 4 cells for weno7js and the hccs family, 3 for
 // the WENO5 family, 2 for weno3js, 1 for upwind1st

@@ -147,15 +147,17 @@ cudaError_t launch_inviscid(int scheme, int dir, int variant, const BoxDev *boxe
                             const WorkItem *items, int nitems, int in_slot, int accumulate,
                             int prim_mode, cudaStream_t st);
 // Marching y and z sweeps (march_kernels.cu) of the FP64 WENO5-JS / WENO5-Z
-// pairs: a work item is (box, group of 32 lines, first cell), walked in `chunks`
-// chunks of `len` cells, which add to the RHS accumulator.  The autotuner's variant v of such a pair
+// pairs: a work item is (box, group of 32 lines), walked in `chunks` chunks of
+// `len` cells, or (chunks 0) such a group's chunk with its first cell; each adds to
+// the RHS accumulator.  The autotuner's variant v of such a pair
 // is the chunk length kMarchLen[v]: short chunks give small boxes enough
 // teams, long ones re-read less of the chunk's 6-cell overlap (256^3 z: 8 to
 // 128 cells 0.95, 0.78, 0.67, 0.60, 0.57 ms; 97 x 61 x 45: 22, 20, 22, 26, 26 us).
 constexpr int kMarchLen[kInvVariants] = {8, 16, 32, 64, 128};
 // The FP64 x sweeps of weno5js, weno5z and weno7js (xsweep_kernels.cu): a work
-// item is (box, group of 16 lines, first cell), walked in `chunks` chunks of
-// `tiles` tiles of 32 cells, a block each; variant v: kXTiles[v].
+// item is (box, group of 16 lines), walked in `chunks` chunks of `tiles` tiles of 32
+// cells, a block each, or (chunks 0) such a group's chunk with its first cell;
+// variant v: kXTiles[v].
 constexpr int kXTiles[kInvVariants] = {1, 2, 4, 8, 16};
 constexpr int kMarchLines = 32, kXLines = 16;
 constexpr bool marched(int scheme, int dir, bool mixed) {

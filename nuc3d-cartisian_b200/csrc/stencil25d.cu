@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(TX *TY, 2) k_visc_flux25(const BoxDev *__restr
     B *const vbase = fieldV<B>(bd, 0);
     const int nx = bp.n[0], ny = bp.n[1], nz = bp.n[2];
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-    const int i0 = it.a * TX, j0 = it.b * TY, k0 = it.c * depth;
+    const int i0 = it.a * TX, j0 = it.b * TY, k0 = warp_uniform(it.c * depth);
     const int i = i0 + tx, j = j0 + ty;
     const bool active = i < nx && j < ny;
     const long long sz = bp.stride[2];

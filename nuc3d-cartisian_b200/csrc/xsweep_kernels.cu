@@ -141,11 +141,12 @@ struct XGeom {
 
 }  // namespace
 
-// Work item (box, group of 16 lines, first cell); blockIdx.y: the chunk of `tiles`
-// tiles from there.
+// Work item (box, group of 16 lines, first cell of a chunk of `tiles` tiles where
+// LISTED, else blockIdx.y is the chunk: a cell read from the item costs the weno7js
+// kernel spills, 192 x 96 x 80 177.7 -> 180.2 us).
 // The primitives are recovered from the state and W is written for the tile's
 // own cells; PM 2: their eigenvalues are folded into the box's maxima as well.
-template <int SCHEME, int PM>
+template <int SCHEME, int PM, bool LISTED>
 __global__ void __launch_bounds__(kThreads, SCHEME == SCHEME_W7 ? 3 : 4)
     k_xsweep(const BoxDev *__restrict__ boxes, const WorkItem *__restrict__ items, int in_slot,
              int tiles) {
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(kThreads, SCHEME == SCHEME_W7 ? 3 : 4)
     const BoxDev &bd = boxes[it.box];
     const BoxParams &bp = bd.p;
     const int n = bp.n[0];
-    const int first = it.b + blockIdx.y * tiles * TC;
+    const int first = LISTED ? it.b : blockIdx.y * tiles * TC;
     if (!bd.active) return;
     const long long np = bd.np;
     const int nlines = bp.n[1] * bp.n[2], L0 = it.a * TL;
@@ -282,24 +283,25 @@ __global__ void __launch_bounds__(kThreads, SCHEME == SCHEME_W7 ? 3 : 4)
 namespace {
 using XSweep = void (*)(const BoxDev *, const WorkItem *, int, int);
 template <int SCHEME>
-XSweep xsweep_pm(int prim_mode) {
-    return prim_mode == 2 ? k_xsweep<SCHEME, 2> : k_xsweep<SCHEME, 1>;
+XSweep xsweep_pm(int prim_mode, bool listed) {
+    if (listed) return prim_mode == 2 ? k_xsweep<SCHEME, 2, true> : k_xsweep<SCHEME, 1, true>;
+    return prim_mode == 2 ? k_xsweep<SCHEME, 2, false> : k_xsweep<SCHEME, 1, false>;
 }
-XSweep xsweep_kernel(int scheme, int prim_mode, size_t &smem) {
+XSweep xsweep_kernel(int scheme, int prim_mode, bool listed, size_t &smem) {
     smem = scheme == SCHEME_W7  ? XGeom<SCHEME_W7>::SMEM
            : scheme == SCHEME_Z ? XGeom<SCHEME_Z>::SMEM
                                 : XGeom<SCHEME_JS>::SMEM;
-    return scheme == SCHEME_JS  ? xsweep_pm<SCHEME_JS>(prim_mode)
-           : scheme == SCHEME_Z ? xsweep_pm<SCHEME_Z>(prim_mode)
-                                : xsweep_pm<SCHEME_W7>(prim_mode);
+    return scheme == SCHEME_JS  ? xsweep_pm<SCHEME_JS>(prim_mode, listed)
+           : scheme == SCHEME_Z ? xsweep_pm<SCHEME_Z>(prim_mode, listed)
+                                : xsweep_pm<SCHEME_W7>(prim_mode, listed);
 }
 }  // namespace
 
 cudaError_t prepare_xsweep_kernels() {
     for (int s : {SCHEME_JS, SCHEME_Z, SCHEME_W7})
-        for (int m = 1; m < 3; ++m) {
+        for (int m = 0; m < 4; ++m) {
             size_t smem;
-            const XSweep k = xsweep_kernel(s, m, smem);
+            const XSweep k = xsweep_kernel(s, 1 + m % 2, m / 2 == 1, smem);
             cudaError_t e =
                 cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return e;
@@ -311,8 +313,8 @@ cudaError_t launch_xsweep(int scheme, const BoxDev *boxes, const WorkItem *items
                           int chunks, int in_slot, int tiles, int prim_mode, cudaStream_t st) {
     if (nitems <= 0) return cudaSuccess;
     size_t smem;
-    const XSweep k = xsweep_kernel(scheme, prim_mode, smem);
-    k<<<dim3(nitems, chunks), kThreads, smem, st>>>(boxes, items, in_slot, tiles);
+    const XSweep k = xsweep_kernel(scheme, prim_mode, chunks == 0, smem);
+    k<<<dim3(nitems, chunks > 0 ? chunks : 1), kThreads, smem, st>>>(boxes, items, in_slot, tiles);
     return cudaGetLastError();
 }
 
