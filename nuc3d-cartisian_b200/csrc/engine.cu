@@ -1030,7 +1030,8 @@ int Engine::autotune() {
                              : launch_update_classes<double>(v, sa, stream_);
             });
             pencil_tune_ms[v] = ms;
-            if (ms < pencil_tune_ms[best]) best = v;
+            const double gain = v >= kLongPencils && best < kLongPencils ? kShortPencilGain : 1.0;
+            if (ms < gain * pencil_tune_ms[best]) best = v;
         }
         pencil_variant = best;
         kept_pencil = (signed char)best;
