@@ -203,9 +203,9 @@ private:
     static constexpr long long kPencilShortBlocks = 600;
     // Short depths are gone into only if the pass at 8 planes is this much faster
     // than at 16.  Where they tie, the short one loses in the step, whose sweeps run
-    // beside the viscous fluxes and share HBM with its deeper halos: 160 x 100 x 60
-    // FP64 1478 against 1450 us at 16 planes, 90 x 150 x 70 hccs mixed 3512 against
-    // 3478.  Boxes that the short depths are for gain 10 to 50 % of the pass.
+    // beside the viscous fluxes and share HBM with its deeper halos: two steps of
+    // 160 x 100 x 60 FP64 1478 against 1450 us at 16 planes, of 90 x 150 x 70 hccs
+    // mixed 3512 against 3478.  Boxes that the short depths are for gain 10 to 50 % of the pass.
     static constexpr double kShortPencilGain = 0.97;
     int pv() const { return pencil_variant < 0 ? 0 : pencil_variant; }
     // Mixed precision stages each line's split fluxes as FP32 offsets from
